@@ -107,7 +107,9 @@ __device__ __forceinline__ void halley_bisect_update_generic(HalleyState& s, flo
 template <int MAXB>
 __device__ __forceinline__ float hist_tau_alpha15(const int* cnt, int bins, float tau0) {
   float sz = 1.f, sn = 1.f, szz = 1.f;
-  for (int sj = bins - 1; sj >= 0; --sj) {
+#pragma unroll   // (fixed trip count: `cnt` stays in registers)
+  for (int sj = MAXB - 1; sj >= 0; --sj) {
+    if (sj >= bins) continue;
     float c = (float)(cnt[sj] - (sj == bins - 1 ? 1 : 0));
     float e = (float)sj / (float)bins;
     float nzz = szz + c * (e * e);

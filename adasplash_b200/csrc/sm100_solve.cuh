@@ -32,9 +32,21 @@
 // histogram covers [tau0, tau0 + 1], and tau never falls below tau0 (the largest
 // probability (z_max - tau)^2 is at most 1).  Those scores are a tiny part of a
 // row, so the kernel computes S twice, not (3 + niter) times: sweep 1 finds the
-// row maxima; sweep 2 appends every score >= tau0 (value and key index)
+// row maxima; sweep 2 appends every score that can matter (value and key index)
 // to a per-thread list in a shared-memory pool; the histogram, the Halley steps
-// and the final bitmap + step run on the lists.  The counts and bitmap bits are
+// and the final bitmap + step run on the lists.
+//
+// Which scores can matter: sweep 1 keeps, for the price of one maximum, sixteen maxima
+// per thread (one per pair of the 32 columns it reads at a time), i.e. 32 different
+// scores of the row.  The histogram's lower bound of tau is monotone in the set it is
+// taken over, so the bound from these 32 scores is at most the bound from the whole row;
+// the row's own bound looks only at bins above itself and no later step goes below it.
+// So sweep 2 lists the scores above the bound of the 32: 9 per row instead of the 21
+// within 1 of the maximum at N = 8192 with inputs of spread 1.5, 58 instead of 500 at
+// N = 16384 with unit-variance inputs -- which used to overflow the pool.  Measured:
+// 2 x 16 heads, N = 8192, D = 128: 807 -> 643 us; 2 x 32 heads on 8, N = 16384, unit
+// variance: 15.5 -> 8.7 ms.
+//  The counts and bitmap bits are
 // the same integers either way; the Halley sums add the same terms in list order.
 // If the pool fills up (rows whose scores are nearly flat), sweep 2 goes on as a
 // plain histogram sweep for the scores that find no room, and the CTA sweeps S
@@ -62,6 +74,7 @@ constexpr int kSolveTmemCols = 512;  // three S buffers at columns 0 / 128 / 256
 constexpr uint32_t kSolveQCol = 384;
 constexpr int kSolveBufs = 3;
 constexpr int kSolveRows = 2 * kBlockM;  // query rows per CTA
+constexpr int kSolveClasses = 16;        // maxima a row thread keeps: one per pair of the 32 columns it reads at a time
 
 enum SweepMode : int { kModeMax = 0, kModeHist = 1, kModeHalley = 2, kModeFinal = 3, kModeCollect = 4, kModeRecollect = 5 };
 
@@ -356,6 +369,10 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     }
 
     float mx = -1.0e3f, tau0 = 0.f;
+    float cls[kSolveClasses];  // maxima of this thread's keys by position (see below)
+#pragma unroll
+    for (int c = 0; c < kSolveClasses; ++c) cls[c] = -1.0e3f;
+    float thr_list = 0.f;      // scores from here on go to the lists
     int cnt[8];
     HalleyState hs;
     hs.t = hs.lo = hs.hi = 0.f;
@@ -413,7 +430,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         // Collecting takes scores from a hair below tau0: a Halley step may land up to 1e-5
         // below its bracket, and a sweep over S would then see those scores too.  The
         // histogram over the list tests each score against tau0 itself.
-        const float thr = mode == kModeCollect ? tau0 - 2e-5f - margin : ((V1 && mode == kModeFinal) ? hs.lo : hs.t);
+        const float thr = mode == kModeCollect ? thr_list - margin : ((V1 && mode == kModeFinal) ? hs.lo : hs.t);
         // (Register budget: the kernel keeps nearly all of the SM's shared memory, which leaves
         // almost no L1 for local memory -- a spill in this loop costs an L2 round trip.)
 #pragma unroll 1
@@ -435,16 +452,10 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
             for (int c = 0; c < 32; ++c) v[c] = (c <= lim) ? v[c] : kMaskedScore;
           }
           if (mode == kModeMax) {
-            // four independent chains: a single running max would serialise the dependent ops
-            float m0_ = mx, m1_ = mx, m2_ = mx, m3_ = mx;
+            // one maximum per pair of columns: as many instructions as a single maximum takes,
+            // and the sixteen values are sixteen different scores of the row
 #pragma unroll
-            for (int c = 0; c < 32; c += 8) {
-              m0_ = ptx::fmax3(m0_, v[c], v[c + 1]);
-              m1_ = ptx::fmax3(m1_, v[c + 2], v[c + 3]);
-              m2_ = ptx::fmax3(m2_, v[c + 4], v[c + 5]);
-              m3_ = ptx::fmax3(m3_, v[c + 6], v[c + 7]);
-            }
-            mx = fmaxf(fmaxf(m0_, m1_), fmaxf(m2_, m3_));
+            for (int c = 0; c < kSolveClasses; ++c) cls[c] = ptx::fmax3(cls[c], v[2 * c], v[2 * c + 1]);
           } else if (mode == kModeCollect) {
             // The histogram sweep: every score within 1 of the row maximum goes to this
             // thread's list while the pool has room (and is binned from there after the
@@ -626,7 +637,8 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         int bins_cnt[8], cum[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) cum[c] = cnt[c] + __float_as_int(o[c]);
-        for (int c = 0; c < p.bins; ++c) bins_cnt[c] = cum[c] - (c + 1 < p.bins ? cum[c + 1] : 0);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) bins_cnt[c] = cum[c] - (c + 1 < 8 && c + 1 < p.bins ? cum[c + 1 < 8 ? c + 1 : 7] : 0);
         const float t1 = hist_tau_alpha15<8>(bins_cnt, p.bins, tau0);
         hs.lo = t1;
         hs.hi = t1 + 1.0f / fbins;
@@ -661,7 +673,24 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
       if (grp_on) {
         reset_stats();
         sweep_tiles(std::integral_constant<int, kModeMax>{});
+#pragma unroll
+        for (int c = 0; c < kSolveClasses; ++c) mx = fmaxf(mx, cls[c]);
         exchange(kModeMax);
+        thr_list = tau0 - 2e-5f;
+        if constexpr (!V1) {
+          // the histogram of the row's 32 class maxima alone: its lower bound of tau is a lower
+          // bound of the whole row's
+#pragma unroll
+          for (int c = 0; c < kSolveClasses; ++c) {
+            const float prj = (cls[c] - tau0) * fbins;
+            const int bsel = prj >= 0.f ? min(__float2int_rd(prj), 7) : -1;
+#pragma unroll
+            for (int bb = 0; bb < 8; ++bb) cnt[bb] += (bb <= bsel) ? 1 : 0;
+          }
+          exchange(kModeHist);
+          thr_list = fmaxf(thr_list, hs.lo - 2e-5f);
+          reset_stats();
+        }
         sweep_tiles(std::integral_constant<int, kModeCollect>{});
         if (lane == 0) pool_used[warp] = my_used;
         __syncwarp();
@@ -732,6 +761,14 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           }
         }
         __syncwarp();
+        // Most entries find their tile's bit set already (64 rows share it), so look before the
+        // atomic: hundreds of threads otherwise queue up on a handful of words (64 of 71 us of a
+        // 256-row problem).
+        volatile uint32_t* row_bits = s_bits + (grp * 2 + rb) * p.n_words;
+        auto mark_tile = [&](int kb) {
+          const uint32_t bit = 1u << (kb & 31);
+          if (!(row_bits[kb >> 5] & bit)) atomicOr(const_cast<uint32_t*>(row_bits) + (kb >> 5), bit);
+        };
         for (int it = 0; it <= p.niter; ++it) {
           const bool last = it == p.niter;
           reset_stats();
@@ -741,7 +778,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
               // sub-tiles that hold a score above the lower end of the bracket
               if (last) {
                 const int kb = c.key >> kb_shift;
-                if (c.z > hs.lo && row_ok) atomicOr(&s_bits[(grp * 2 + rb) * p.n_words + (kb >> 5)], 1u << (kb & 31));
+                if (c.z > hs.lo && row_ok) mark_tile(kb);
               } else {
                 const float d = c.z - hs.t;
                 if (d > 0.f) {
@@ -759,7 +796,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
                 // the final step also records the 64x64 sub-tiles that hold a score above the
                 // tau entering it (row block rb of this group, key block c.kb)
                 const int kb = c.key >> kb_shift;
-                if (last && row_ok) atomicOr(&s_bits[(grp * 2 + rb) * p.n_words + (kb >> 5)], 1u << (kb & 31));
+                if (last && row_ok) mark_tile(kb);
               }
             }
           };
