@@ -7,6 +7,15 @@
 // 16x16 grid holds rows ty+16i and columns tx+16j (i,j < 4).  Operand tiles
 // live in shared memory as fp32 with a row pitch of D+4 floats so that the
 // float4 reads of the inner product are conflict-free.
+//
+// What bounds them: a tile product is 64x64xD multiply-adds, 2048 clocks of an SM's fp32 pipe at
+// D = 64, and the float4 operand reads from shared memory keep about three quarters of that
+// time busy beside it.  So every operand is read in float4 (or, for the staged weights, a float4
+// of four consecutive positions), the multiply-adds are the packed two-lane ones (half the issue
+// slots; the same fp32 arithmetic), and the tiles of fp32 inputs arrive by cp.async while the
+// product before them runs.  Row blocks are handed out heaviest first over all heads: a causal
+// problem of a few heads is as long as its last row block.  fp32, 8 heads of N = 2048, D = 64, unit
+// variance, forward and backward: 2.11 -> 0.96 ms (solver 619, forward 466, dQ 425, dK/dV 615 us before).
 #pragma once
 #include "common.cuh"
 
@@ -14,12 +23,28 @@ namespace ads {
 namespace simt {
 
 constexpr int kThreads = 256;
-constexpr int kPPitch = 65;  // pitch of the 64x64 P / dS staging tiles
+constexpr int kPPitch = 80;  // pitch of the 64x64 P / dS staging tiles: rows 16-byte aligned, two neighbours 16 banks apart
 
 template <int D> struct Cfg {
   static constexpr int pitch = D + 4;
   static constexpr int tile_floats = 64 * pitch;
-  static constexpr int dcols = D / 16;  // output columns per thread
+  static constexpr int dcols = D / 16;  // output columns per thread: runs of `vw` adjacent ones
+  static constexpr int vw = dcols < 4 ? dcols : 4;
+  // room for the streamed operand tiles side by side (head dim 256: one buffer, used in turn)
+  static constexpr bool split = D <= 128;
+  // column c (0 .. dcols-1) of the thread at tx
+  static __device__ __forceinline__ int col(int tx, int c) { return (c / vw) * 16 * vw + tx * vw + c % vw; }
+};
+
+// Row block and (batch, head) of this CTA: heaviest row blocks first over all heads.
+struct BlockOf {
+  int m, h, b;
+  __device__ __forceinline__ BlockOf(int nb, int heads, int B, bool descending) {
+    const int bh = blockIdx.x % (heads * B), i = blockIdx.x / (heads * B);
+    m = descending ? nb - 1 - i : i;
+    h = bh % heads;
+    b = bh / heads;
+  }
 };
 
 struct Idx {
@@ -60,15 +85,40 @@ __device__ __forceinline__ void load_tile(float* s, const T* g, int row0, int li
   }
 }
 
+// The same tile, unscaled, on its way: cp.async for fp32 (the caller commits and waits), a plain
+// load for the 16-bit types, which are converted.
+template <typename T, int D>
+__device__ __forceinline__ void stage_tile(float* s, const T* g, int row0, int limit) {
+  if constexpr (sizeof(T) == 4) {
+    constexpr int P = Cfg<D>::pitch;
+    constexpr int VPR = D / 4;
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < 64 * VPR; idx += kThreads) {
+      const int r = idx / VPR, c4 = (idx % VPR) * 4;
+      const bool in = row0 + r < limit;
+      const T* src = g + (size_t)(in ? row0 + r : 0) * D + c4;   // rows beyond the limit: zero-filled, nothing read
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s + r * P + c4);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+    }
+  } else {
+    load_tile<T, D, false>(s, g, row0, limit, 1.0f);
+  }
+}
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void stage_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
 // acc[i][j] = <A[ty+16i, :], B[tx+16j, :]>
 template <int D>
 __device__ __forceinline__ void tile_dot(const float* sA, const float* sB, const Idx& id,
                                          float acc[4][4]) {
   constexpr int P = Cfg<D>::pitch;
+  float2 a2[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) a2[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 4
   for (int d = 0; d < D; d += 4) {
     float4 a[4], b[4];
@@ -80,12 +130,14 @@ __device__ __forceinline__ void tile_dot(const float* sA, const float* sB, const
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-        acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-        acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        a2[i][j] = __ffma2_rn(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), a2[i][j]);
+        a2[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), a2[i][j]);
       }
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = a2[i][j].x + a2[i][j].y;
 }
 
 // The masked score tile of adasplash_v2.py:93-119: keep z where col <= row and
@@ -120,43 +172,62 @@ __device__ __forceinline__ int row16_sumi(int v) {
   return v;
 }
 
-// out[i][c] += sum_j sP[(ty+16i)][j] * sV[j][tx+16c]   (P row-major 64x64, pitch 65)
+// out[i][c] += p[i] * (this thread's columns of one row of X)
 template <int D>
-__device__ __forceinline__ void tile_pv(const float* sP, const float* sV, const Idx& id,
-                                        float (*out)[Cfg<D>::dcols]) {
-  constexpr int P = Cfg<D>::pitch;
-  constexpr int DC = Cfg<D>::dcols;
-#pragma unroll 2
-  for (int j = 0; j < 64; ++j) {
-    float p[4], v[DC];
+__device__ __forceinline__ void row_axpy(const float (&p)[4], const float* xrow, int tx, float (*out)[Cfg<D>::dcols]) {
+  constexpr int DC = Cfg<D>::dcols, VW = Cfg<D>::vw;
+  float v[DC];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = sP[(id.ty + 16 * i) * kPPitch + j];
+  for (int c = 0; c < DC; c += VW) {
+    const float* src = xrow + Cfg<D>::col(tx, c);
+    if constexpr (VW == 4) *reinterpret_cast<float4*>(v + c) = *reinterpret_cast<const float4*>(src);
+    else if constexpr (VW == 2) *reinterpret_cast<float2*>(v + c) = *reinterpret_cast<const float2*>(src);
+    else v[c] = *src;
+  }
 #pragma unroll
-    for (int c = 0; c < DC; ++c) v[c] = sV[j * P + id.tx + 16 * c];
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (VW >= 2) {
+      const float2 pp = make_float2(p[i], p[i]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int c = 0; c < DC; c += 2) {
+        const float2 r = __ffma2_rn(pp, make_float2(v[c], v[c + 1]), make_float2(out[i][c], out[i][c + 1]));
+        out[i][c] = r.x; out[i][c + 1] = r.y;
+      }
+    } else {
 #pragma unroll
       for (int c = 0; c < DC; ++c) out[i][c] = fmaf(p[i], v[c], out[i][c]);
+    }
   }
 }
 
-// out[i][c] += sum_q sP[q][(ty+16i)] * sX[q][tx+16c]   (transposed use of the staging tile)
+// out[i][c] += sum_j sP[ty+16i][j] * sV[j][col(c)]   (P row-major 64x64)
+template <int D>
+__device__ __forceinline__ void tile_pv(const float* sP, const float* sV, const Idx& id,
+                                        float (*out)[Cfg<D>::dcols]) {
+#pragma unroll 2
+  for (int j = 0; j < 64; j += 4) {
+    float4 p[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(sP + (id.ty + 16 * i) * kPPitch + j);
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      float pj[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pj[i] = jj == 0 ? p[i].x : (jj == 1 ? p[i].y : (jj == 2 ? p[i].z : p[i].w));
+      row_axpy<D>(pj, sV + (j + jj) * Cfg<D>::pitch, id.tx, out);
+    }
+  }
+}
+
+// out[i][c] += sum_q sP[q][4ty+i] * sX[q][col(c)]   (transposed use of the staging tile)
 template <int D>
 __device__ __forceinline__ void tile_ptx(const float* sP, const float* sX, const Idx& id,
                                          float (*out)[Cfg<D>::dcols]) {
-  constexpr int P = Cfg<D>::pitch;
-  constexpr int DC = Cfg<D>::dcols;
-#pragma unroll 2
+#pragma unroll 4
   for (int q = 0; q < 64; ++q) {
-    float p[4], v[DC];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = sP[q * kPPitch + id.ty + 16 * i];
-#pragma unroll
-    for (int c = 0; c < DC; ++c) v[c] = sX[q * P + id.tx + 16 * c];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < DC; ++c) out[i][c] = fmaf(p[i], v[c], out[i][c]);
+    const float4 p4 = *reinterpret_cast<const float4*>(sP + q * kPPitch + 4 * id.ty);
+    const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+    row_axpy<D>(p, sX + q * Cfg<D>::pitch, id.tx, out);
   }
 }
 
@@ -206,16 +277,41 @@ struct Params {
 
 // ---------------------------------------------------------------------------
 // Solver: row max -> histogram lower bound -> Halley refinements -> bitmap.
-// One launch performs all sweeps; the scaled Q tile stays in shared memory and
-// the K tiles are re-streamed (they are L2 resident per head).
+// One launch, two sweeps over S: the scaled Q tile stays in shared memory, the K tiles are
+// streamed (they are L2 resident per head).
+//
+// Everything after the row maximum looks only at scores above a lower bound of tau, which are few.
+// Sweep 1 keeps the maximum of each of a row's 64 column classes (key mod 64), i.e. 64 different
+// scores; the histogram bound is monotone in the set it is taken over, so the bound from those
+// is a lower bound of the row's, and the row's own bound reads no bin below itself.  Sweep 2
+// lists the scores above it (minus the 1e-5 a step may undercut its bracket by) in a fixed order,
+// and the histogram, the steps and the block mask run on the lists.  First-generation calls have no
+// histogram: their lists hold the scores within 1 of the maximum.  A CTA with a row that has more
+// than kSolveList of them sweeps S for every step.
 // ---------------------------------------------------------------------------
+constexpr int kSolveList = 128;  // listed scores per row
+
+template <int D>
+struct SolveSmem {
+  static constexpr int k_bufs = Cfg<D>::split ? 2 : 1;
+  static constexpr int list_off = (1 + k_bufs) * Cfg<D>::tile_floats;           // floats
+  static constexpr int tile_off = list_off + 64 * kSolveList;                   // uint16: key tile of each listed score
+  static constexpr int bits_off = tile_off + 64 * kSolveList / 2;
+  static size_t bytes(int n_words) { return ((size_t)bits_off + n_words) * sizeof(float); }
+};
+
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
   extern __shared__ __align__(16) float smem[];
+  using L = SolveSmem<D>;
   float* sQ = smem;
   float* sK = smem + Cfg<D>::tile_floats;
+  float* s_list = smem + L::list_off;
+  uint16_t* s_tile = reinterpret_cast<uint16_t*>(smem + L::tile_off);
+  uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem + L::bits_off);
   const Idx id;
-  const int m = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const BlockOf blk(p.nb, p.Hq, p.B, true);
+  const int m = blk.m, h = blk.h, b = blk.b;
   const int len = load_len(p.varlen, p.varlen_is_i64, b, p.N);
   const int m0 = m * kTile;
   if (m0 >= len) return;
@@ -226,6 +322,7 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
   int32_t* bm = p.bmask + (((size_t)b * p.Hq + h) * p.rows_padded + m) * (size_t)p.n_words;
   const float sc = p.zscale;
   load_tile<T, D, true>(sQ, qg, m0, len, sc);
+  for (int w = threadIdx.x; w < p.n_words; w += kThreads) s_bits[w] = 0u;
   const bool causal = p.causal != 0;
   const bool v2_path = causal && p.alpha == 1.5f;  // the reference's AdaSplash-2 trajectory
   const int up_to = causal ? min(m0 + kTile, len) : len;
@@ -234,29 +331,122 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
   HalleyState st[4];
 
   auto sweep = [&](auto&& per_tile) {
+    __syncthreads();  // the buffers of the sweep before are free
+    stage_tile<T, D>(sK, kg, 0, len);
+    stage_commit();
     for (int n = 0; n < ntiles; ++n) {
-      __syncthreads();
-      load_tile<T, D, false>(sK, kg, n * kTile, len, 1.0f);
-      __syncthreads();
-      tile_dot<D>(sQ, sK, id, acc);
+      const float* cur = sK + (n % L::k_bufs) * Cfg<D>::tile_floats;
+      stage_wait<0>();
+      __syncthreads();  // tile n is here, and everyone is through with tile n - 1
+      if (L::k_bufs > 1 && n + 1 < ntiles) {
+        stage_tile<T, D>(sK + ((n + 1) % L::k_bufs) * Cfg<D>::tile_floats, kg, (n + 1) * kTile, len);
+        stage_commit();
+      }
+      tile_dot<D>(sQ, cur, id, acc);
+      if (L::k_bufs == 1) {
+        __syncthreads();
+        if (n + 1 < ntiles) { stage_tile<T, D>(sK, kg, (n + 1) * kTile, len); stage_commit(); }
+      }
       mask_scores(acc, id, m0, n * kTile, len, causal);
       per_tile(n);
     }
   };
+  // histogram of z - tau0 on [0,1] (adasplash_v2.py:387-431) as cumulative counts
+  // N_b = #{(z - tau0) * BINS >= b}, and the bracket it gives
+  auto bracket = [&](HalleyState& s, int (&cnt)[8], float tau0) {
+    int bins_cnt[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) cnt[c] = row16_sumi(cnt[c]);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) bins_cnt[c] = cnt[c] - (c + 1 < 8 && c + 1 < p.bins ? cnt[c + 1 < 8 ? c + 1 : 7] : 0);
+    const float t1 = hist_tau_alpha15<8>(bins_cnt, p.bins, tau0);
+    s.lo = t1;
+    s.hi = t1 + 1.0f / (float)p.bins;
+    s.t = 0.5f * (s.lo + s.hi);
+  };
+  auto count = [&](int (&cnt)[8], float z, float tau0) {
+    const float pr = (z - tau0) * (float)p.bins;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) cnt[c] += (pr >= (float)c) ? 1 : 0;
+  };
 
+  bool listed = false;
+  int n_list[4] = {0, 0, 0, 0};   // listed scores of this thread's rows
   if (!p.tau_given) {
-    // sweep 1: row maximum (adasplash_v2.py:236-266)
-    float mx[4] = {-1.0e3f, -1.0e3f, -1.0e3f, -1.0e3f};
-    sweep([&](int) {
+    float tau0[4], thr[4];
+    {
+      // sweep 1: row maximum (adasplash_v2.py:236-266), by column class
+      float mx[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mx[i] = fmaxf(mx[i], acc[i][j]);
-    });
-    float tau0[4];
+        for (int j = 0; j < 4; ++j) mx[i][j] = -INFINITY;
+      sweep([&](int) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tau0[i] = row16_max(mx[i]) - 1.0f;
-    if (!v2_path) {
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) mx[i][j] = fmaxf(mx[i][j], acc[i][j]);
+      });
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float m4 = fmaxf(fmaxf(mx[i][0], mx[i][1]), fmaxf(mx[i][2], mx[i][3]));
+        tau0[i] = fmaxf(row16_max(m4), -1.0e3f) - 1.0f;
+        thr[i] = tau0[i] - 2e-5f;
+        if (v2_path) {
+          int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) count(cnt, mx[i][j], tau0[i]);
+          bracket(st[i], cnt, tau0[i]);
+          thr[i] = fmaxf(thr[i], st[i].lo - 2e-5f);
+        }
+      }
+    }
+    // sweep 2: lists.  The sixteen threads of a row take their slots from a vote.
+    sweep([&](int n) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int rr = id.ty + 16 * i;
+        const bool row_ok = m0 + rr < len;
+        const float m4 = fmaxf(fmaxf(acc[i][0], acc[i][1]), fmaxf(acc[i][2], acc[i][3]));
+        if (!__any_sync(0xffffffffu, row_ok && m4 >= thr[i])) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool want = row_ok && acc[i][j] >= thr[i];
+          const uint32_t votes = (__ballot_sync(0xffffffffu, want) >> (threadIdx.x & 16)) & 0xffffu;
+          if (want) {
+            const int k = n_list[i] + __popc(votes & ((1u << id.tx) - 1u));
+            if (k < kSolveList) {
+              s_list[rr * kSolveList + k] = acc[i][j];
+              s_tile[rr * kSolveList + k] = (uint16_t)n;
+            }
+          }
+          n_list[i] += __popc(votes);
+        }
+      }
+    });
+    const bool over = max(max(n_list[0], n_list[1]), max(n_list[2], n_list[3])) > kSolveList || ntiles > 65536;
+    listed = !__syncthreads_or(over);
+    if (v2_path) {
+      int cnt[4][8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) cnt[i][c] = 0;
+      if (listed) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          for (int e = id.tx; e < n_list[i]; e += 16) count(cnt[i], s_list[(id.ty + 16 * i) * kSolveList + e], tau0[i]);
+      } else {
+        sweep([&](int) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) count(cnt[i], acc[i][j], tau0[i]);
+        });
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bracket(st[i], cnt[i], tau0[i]);
+    } else {
       // generic alpha / non-causal (adasplash_block_mask.py:170-176): bracket
       // [max - 1, max - n^(1-alpha)], start at its midpoint
 #pragma unroll
@@ -267,36 +457,6 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
         st[i].hi = tau0[i] + 1.0f - exp2f((1.0f - p.alpha) * log2f(n));
         st[i].t = 0.5f * (st[i].lo + st[i].hi);
       }
-    } else {
-    // sweep 2: histogram of z - tau0 on [0,1] (adasplash_v2.py:387-431), as
-    // cumulative counts N_b = #{(z - tau0) * BINS >= b}
-    int cnt[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) cnt[i][c] = 0;
-    const float fb = (float)p.bins;
-    sweep([&](int) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float pr = (acc[i][j] - tau0[i]) * fb;
-#pragma unroll
-          for (int c = 0; c < 8; ++c) cnt[i][c] += (pr >= (float)c) ? 1 : 0;
-        }
-    });
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int bins_cnt[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) cnt[i][c] = row16_sumi(cnt[i][c]);
-      for (int c = 0; c < p.bins; ++c) bins_cnt[c] = cnt[i][c] - (c + 1 < p.bins ? cnt[i][c + 1] : 0);
-      float t1 = hist_tau_alpha15<8>(bins_cnt, p.bins, tau0[i]);
-      st[i].lo = t1;
-      st[i].hi = t1 + 1.0f / fb;
-      st[i].t = 0.5f * (st[i].lo + st[i].hi);
-    }
     }
   } else {
 #pragma unroll
@@ -306,9 +466,9 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
       st[i].lo = st[i].hi = st[i].t;
     }
   }
-  // refinement sweeps; the last one also records the bitmap for the tau that
+  // refinement steps; the last one also records the bitmap for the tau that
   // enters it (adasplash_v2.py:567-675)
-  // Generic path: niter updates, then a bitmap-only sweep at the lower end of the
+  // Generic path: niter updates, then a bitmap-only step at the lower end of the
   // bracket (tau_lo <= tau*, so no tile of the support can be missed).
   const Powers pw(p.alpha);
   const int total = p.tau_given ? 1 : p.niter + 1;
@@ -316,43 +476,44 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
     const bool last = (it == total - 1);
     const bool bitmap_only = last && !v2_path && !p.tau_given;
     float a0[4] = {0, 0, 0, 0}, a1[4] = {0, 0, 0, 0}, a2[4] = {0, 0, 0, 0};
-    uint32_t cur = 0u;  // bitmap word under construction (thread 0 only)
-    sweep([&](int n) {
-      int hit = 0;
+    // one score of row i, in key tile n
+    auto visit = [&](int i, float z, int n) {
+      // rows at or beyond len carry q = 0 and never count as hits
+      const bool row_ok = (m0 + id.ty + 16 * i) < len;
+      const float thr = bitmap_only ? st[i].lo : st[i].t;
+      if (z > thr) {
+        const float u = z - thr;
+        if (pw.mode == 0) {
+          a0[i] = fmaf(u, u, a0[i]);
+          a1[i] += u;
+          a2[i] += 1.f;
+        } else {
+          const float g = pw.g(u);
+          a0[i] += pw.p(u);
+          a1[i] += g;
+          a2[i] += (pw.mode == 2) ? g / u : 0.f;
+        }
+        if (last && row_ok) {
+          const uint32_t bit = 1u << (n & 31);
+          if (!(*(volatile uint32_t*)(s_bits + (n >> 5)) & bit)) atomicOr(s_bits + (n >> 5), bit);
+        }
+      }
+    };
+    if (listed) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        // rows at or beyond len carry q = 0 and never count as hits
-        bool row_ok = (m0 + id.ty + 16 * i) < len;
-#pragma unroll
-        const float thr = bitmap_only ? st[i].lo : st[i].t;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          bool mk = acc[i][j] > thr;
-          float u = mk ? (acc[i][j] - thr) : 0.f;
-          if (pw.mode == 0) {
-            a0[i] = fmaf(u, u, a0[i]);
-            a1[i] += u;
-            a2[i] += mk ? 1.f : 0.f;
-          } else if (mk) {
-            const float g = pw.g(u);
-            a0[i] += pw.p(u);
-            a1[i] += g;
-            a2[i] += (pw.mode == 2) ? g / u : 0.f;
-          }
-          hit |= (mk && row_ok) ? 1 : 0;
-        }
+        const int o = (id.ty + 16 * i) * kSolveList;
+        for (int e = id.tx; e < n_list[i]; e += 16) visit(i, s_list[o + e], s_tile[o + e]);
       }
-      if (last) {
-        int any = __syncthreads_or(hit);
-        if (threadIdx.x == 0) {
-          if (any) cur |= (1u << (n & 31));
-          if ((n & 31) == 31 || n == ntiles - 1) {
-            bm[n >> 5] = (int32_t)cur;
-            cur = 0u;
-          }
+    } else {
+      sweep([&](int n) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) visit(i, acc[i][j], n);
         }
-      }
-    });
+      });
+    }
     if (!p.tau_given && !bitmap_only) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -362,6 +523,8 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
       }
     }
   }
+  __syncthreads();  // every bit is set
+  for (int w = threadIdx.x; w < p.n_words; w += kThreads) bm[w] = (int32_t)s_bits[w];
   if (!p.tau_given && id.tx == 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -374,16 +537,34 @@ __global__ void __launch_bounds__(kThreads) solve_kernel(Params p) {
 // ---------------------------------------------------------------------------
 // Sparse forward (adasplash_v2.py:696-835)
 // ---------------------------------------------------------------------------
+// The set bits of one bitmap row, in ascending order (-1: no more).
+struct SetBits {
+  const int32_t* words; int n_words, w; uint32_t cur;
+  __device__ __forceinline__ SetBits(const int32_t* ws, int n) : words(ws), n_words(n), w(0), cur(n > 0 ? (uint32_t)ws[0] : 0u) {}
+  __device__ __forceinline__ int next() {
+    while (cur == 0u) {
+      if (++w >= n_words) { w = n_words; return -1; }
+      cur = (uint32_t)words[w];
+    }
+    const int n = (w << 5) + __ffs(cur) - 1;
+    cur &= cur - 1u;
+    return n;
+  }
+};
+
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) fwd_kernel(Params p) {
   extern __shared__ __align__(16) float smem[];
   constexpr int DC = Cfg<D>::dcols;
+  constexpr bool SPLIT = Cfg<D>::split;
   float* sQ = smem;
-  float* sKV = sQ + Cfg<D>::tile_floats;
-  float* sP = sKV + Cfg<D>::tile_floats;
+  float* sK = sQ + Cfg<D>::tile_floats;
+  float* sV = SPLIT ? sK + Cfg<D>::tile_floats : sK;
+  float* sP = sV + Cfg<D>::tile_floats;
   float* sU = sP + 64 * kPPitch;
   const Idx id;
-  const int m = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const BlockOf blk(p.nb, p.Hq, p.B, true);
+  const int m = blk.m, h = blk.h, b = blk.b;
   const int len = load_len(p.varlen, p.varlen_is_i64, b, p.N);
   const int m0 = m * kTile;
   const size_t qoff = ((size_t)b * p.Hq + h) * (size_t)p.N * D;
@@ -412,33 +593,39 @@ __global__ void __launch_bounds__(kThreads) fwd_kernel(Params p) {
       t[i] = row < len ? tg[row] : 0.f;
     }
     float acc[4][4];
-    for (int w = 0; w < p.n_words; ++w) {
-      uint32_t word = (uint32_t)bm[w];
-      while (word) {
-        int n = (w << 5) + __ffs(word) - 1;
-        word &= word - 1;
-        __syncthreads();
-        load_tile<T, D, false>(sKV, kg, n * kTile, len, 1.0f);
-        __syncthreads();
-        tile_dot<D>(sQ, sKV, id, acc);
-        mask_scores(acc, id, m0, n * kTile, len, p.causal != 0);
-        __syncthreads();
-        load_tile<T, D, false>(sKV, vg, n * kTile, len, 1.0f);
+    SetBits tiles(bm, p.n_words);
+    int n = tiles.next();
+    if (n >= 0) { stage_tile<T, D>(sK, kg, n * kTile, len); stage_commit(); }
+    while (n >= 0) {
+      if (SPLIT) { stage_tile<T, D>(sV, vg, n * kTile, len); stage_commit(); stage_wait<1>(); }
+      else stage_wait<0>();
+      __syncthreads();   // K is here
+      tile_dot<D>(sQ, sK, id, acc);
+      mask_scores(acc, id, m0, n * kTile, len, p.causal != 0);
+      const int n2 = tiles.next();
+      __syncthreads();   // K is free
+      if (!SPLIT) stage_tile<T, D>(sV, vg, n * kTile, len);
+      else if (n2 >= 0) stage_tile<T, D>(sK, kg, n2 * kTile, len);
+      stage_commit();
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float u = fmaxf(acc[i][j] - t[i], 0.f);
-            const float gw = pw.g(u);
-            supp[i] += gw;
-            sP[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(pw.p(u));
-            sU[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(gw);
-          }
-        __syncthreads();
-        tile_pv<D>(sP, sKV, id, o);
-        tile_pv<D>(sU, sKV, id, o2);
-      }
+        for (int j = 0; j < 4; ++j) {
+          const float u = fmaxf(acc[i][j] - t[i], 0.f);
+          const float gw = pw.g(u);
+          supp[i] += gw;
+          sP[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(pw.p(u));
+          sU[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(gw);
+        }
+      if (SPLIT) stage_wait<1>(); else stage_wait<0>();
+      __syncthreads();   // V and the weights are here
+      tile_pv<D>(sP, sV, id, o);
+      tile_pv<D>(sU, sV, id, o2);
+      __syncthreads();   // they are free
+      if (!SPLIT && n2 >= 0) { stage_tile<T, D>(sK, kg, n2 * kTile, len); stage_commit(); }
+      n = n2;
     }
+    stage_wait<0>();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -449,7 +636,7 @@ __global__ void __launch_bounds__(kThreads) fwd_kernel(Params p) {
     float inv = valid ? 1.0f / s : 0.f;
 #pragma unroll
     for (int c = 0; c < DC; ++c) {
-      int d = id.tx + 16 * c;
+      const int d = Cfg<D>::col(id.tx, c);
       og[(size_t)row * D + d] = DT<T>::from_f(valid ? o[i][c] : 0.f);
       o2g[(size_t)row * D + d] = DT<T>::from_f(valid ? o2[i][c] * inv : 0.f);
     }
@@ -554,12 +741,15 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) bwd_dq_kernel(Params p) {
   extern __shared__ __align__(16) float smem[];
   constexpr int DC = Cfg<D>::dcols;
+  constexpr bool SPLIT = Cfg<D>::split;
   float* sQ = smem;
   float* sDO = sQ + Cfg<D>::tile_floats;
-  float* sKV = sDO + Cfg<D>::tile_floats;
-  float* sDS = sKV + Cfg<D>::tile_floats;
+  float* sV = sDO + Cfg<D>::tile_floats;
+  float* sK = SPLIT ? sV + Cfg<D>::tile_floats : sV;
+  float* sDS = sK + Cfg<D>::tile_floats;
   const Idx id;
-  const int m = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const BlockOf blk(p.nb, p.Hq, p.B, true);
+  const int m = blk.m, h = blk.h, b = blk.b;
   const int len = load_len(p.varlen, p.varlen_is_i64, b, p.N);
   const int m0 = m * kTile;
   const size_t qoff = ((size_t)b * p.Hq + h) * (size_t)p.N * D;
@@ -587,30 +777,39 @@ __global__ void __launch_bounds__(kThreads) bwd_dq_kernel(Params p) {
       dl[i] = row < len ? p.delta[toff + row] : 0.f;
     }
     float dp[4][4], acc[4][4];
-    for (int w = 0; w < p.n_words; ++w) {
-      uint32_t word = (uint32_t)bm[w];
-      while (word) {
-        int n = (w << 5) + __ffs(word) - 1;
-        word &= word - 1;
+    SetBits tiles(bm, p.n_words);
+    int n = tiles.next();
+    if (n >= 0) { stage_tile<T, D>(sV, vg, n * kTile, len); stage_commit(); }
+    while (n >= 0) {
+      if (SPLIT) { stage_tile<T, D>(sK, kg, n * kTile, len); stage_commit(); stage_wait<1>(); }
+      else stage_wait<0>();
+      __syncthreads();   // V is here
+      tile_dot<D>(sDO, sV, id, dp);
+      const int n2 = tiles.next();
+      if (SPLIT) stage_wait<0>();
+      __syncthreads();   // V is free; K is here
+      if (SPLIT) {
+        if (n2 >= 0) { stage_tile<T, D>(sV, vg, n2 * kTile, len); stage_commit(); }
+      } else {
+        stage_tile<T, D>(sK, kg, n * kTile, len);
+        stage_commit();
+        stage_wait<0>();
         __syncthreads();
-        load_tile<T, D, false>(sKV, vg, n * kTile, len, 1.0f);
-        __syncthreads();
-        tile_dot<D>(sDO, sKV, id, dp);
-        __syncthreads();
-        load_tile<T, D, false>(sKV, kg, n * kTile, len, 1.0f);
-        __syncthreads();
-        tile_dot<D>(sQ, sKV, id, acc);
-        mask_scores(acc, id, m0, n * kTile, len, p.causal != 0);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float gw = pw.g(fmaxf(acc[i][j] - t[i], 0.f));
-            sDS[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(gw * (dp[i][j] - dl[i]));
-          }
-        __syncthreads();
-        tile_pv<D>(sDS, sKV, id, dq);
       }
+      tile_dot<D>(sQ, sK, id, acc);
+      mask_scores(acc, id, m0, n * kTile, len, p.causal != 0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float gw = pw.g(fmaxf(acc[i][j] - t[i], 0.f));
+          sDS[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(gw * (dp[i][j] - dl[i]));
+        }
+      __syncthreads();   // dS is here
+      tile_pv<D>(sDS, sK, id, dq);
+      __syncthreads();   // K and dS are free
+      if (!SPLIT && n2 >= 0) { stage_tile<T, D>(sV, vg, n2 * kTile, len); stage_commit(); }
+      n = n2;
     }
   }
 #pragma unroll
@@ -620,7 +819,7 @@ __global__ void __launch_bounds__(kThreads) bwd_dq_kernel(Params p) {
     bool valid = row < len;
 #pragma unroll
     for (int c = 0; c < DC; ++c)
-      dqg[(size_t)row * D + id.tx + 16 * c] = DT<T>::from_f(valid ? dq[i][c] * p.sm_scale : 0.f);
+      dqg[(size_t)row * D + Cfg<D>::col(id.tx, c)] = DT<T>::from_f(valid ? dq[i][c] * p.sm_scale : 0.f);
   }
 }
 
@@ -631,12 +830,16 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) bwd_dkv_kernel(Params p) {
   extern __shared__ __align__(16) float smem[];
   constexpr int DC = Cfg<D>::dcols;
+  constexpr bool SPLIT = Cfg<D>::split;
   float* sK = smem;
   float* sV = sK + Cfg<D>::tile_floats;
-  float* sX = sV + Cfg<D>::tile_floats;  // Q, then dO, then Q again
-  float* sP = sX + Cfg<D>::tile_floats;
+  float* sQ = sV + Cfg<D>::tile_floats;
+  float* sDO = SPLIT ? sQ + Cfg<D>::tile_floats : sQ;  // one buffer: Q, then dO, then Q again
+  float* sP = sDO + Cfg<D>::tile_floats;
+  float* sDS = SPLIT ? sP + 64 * kPPitch : sP;
   const Idx id;
-  const int n = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const BlockOf blk(p.nb, p.Hkv, p.B, false);   // causal: the first key tiles see the most rows
+  const int n = blk.m, kvh = blk.h, b = blk.b;
   const int len = load_len(p.varlen, p.varlen_is_i64, b, p.N);
   const int n0 = n * kTile;
   const int G = p.Hq / p.Hkv;
@@ -657,27 +860,59 @@ __global__ void __launch_bounds__(kThreads) bwd_dkv_kernel(Params p) {
       const T* qg = (const T*)p.q + qoff;
       const T* dog = (const T*)p.dout + qoff;
       const int32_t* bt = p.bmask_t + (((size_t)b * p.Hq + h) * p.rows_padded + n) * (size_t)p.n_words;
-      for (int w = 0; w < p.n_words; ++w) {
-        uint32_t word = (uint32_t)bt[w];
-        while (word) {
-          int m = (w << 5) + __ffs(word) - 1;
-          word &= word - 1;
-          const int m0 = m * kTile;
-          float t[4], dl[4];
+      SetBits tiles(bt, p.n_words);
+      int m = tiles.next();
+      if (SPLIT && m >= 0) {
+        stage_tile<T, D>(sDO, dog, m * kTile, len); stage_commit();
+        stage_tile<T, D>(sQ, qg, m * kTile, len); stage_commit();
+      }
+      while (m >= 0) {
+        const int m0 = m * kTile;
+        const int m2 = tiles.next();
+        float t[4], dl[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            int row = m0 + id.ty + 16 * i;
-            t[i] = row < len ? p.taus[toff + row] : 0.f;
-            dl[i] = row < len ? p.delta[toff + row] : 0.f;
-          }
-          float s[4][4], dp[4][4];
+        for (int i = 0; i < 4; ++i) {
+          int row = m0 + id.ty + 16 * i;
+          t[i] = row < len ? p.taus[toff + row] : 0.f;
+          dl[i] = row < len ? p.delta[toff + row] : 0.f;
+        }
+        float s[4][4], dp[4][4];   // [i][j]: q row ty+16i, key tx+16j
+        if constexpr (SPLIT) {
+          stage_wait<1>();
+          __syncthreads();   // dO is here
+          tile_dot<D>(sDO, sV, id, dp);  // dP = dO V^T
+          stage_wait<0>();
+          __syncthreads();   // Q is here
+          tile_dot<D>(sQ, sK, id, s);
+          mask_scores(s, id, m0, n0, len, p.causal != 0);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float u = fmaxf(s[i][j] - t[i], 0.f);
+              sP[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(pw.p(u));
+              sDS[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(pw.g(u) * (dp[i][j] - dl[i]));
+            }
+          __syncthreads();   // P and dS are here
+          tile_ptx<D>(sP, sDO, id, dv);  // dV += P^T dO
+          __syncthreads();   // dO is free
+          if (m2 >= 0) stage_tile<T, D>(sDO, dog, m2 * kTile, len);
+          stage_commit();
+          tile_ptx<D>(sDS, sQ, id, dk);  // dK += dS^T Q
+          __syncthreads();   // Q, P and dS are free
+          if (m2 >= 0) stage_tile<T, D>(sQ, qg, m2 * kTile, len);
+          stage_commit();
+        } else {
           __syncthreads();
-          load_tile<T, D, false>(sX, qg, m0, len, 1.0f);
+          stage_tile<T, D>(sQ, qg, m0, len);
+          stage_commit();
+          stage_wait<0>();
           __syncthreads();
-          tile_dot<D>(sX, sK, id, s);   // s[i][j]: q row ty+16i, key tx+16j
+          tile_dot<D>(sQ, sK, id, s);
           mask_scores(s, id, m0, n0, len, p.causal != 0);
           __syncthreads();
-          load_tile<T, D, false>(sX, dog, m0, len, 1.0f);
+          stage_tile<T, D>(sDO, dog, m0, len);
+          stage_commit();
 #pragma unroll
           for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -686,33 +921,38 @@ __global__ void __launch_bounds__(kThreads) bwd_dkv_kernel(Params p) {
               s[i][j] = pw.g(u);
               sP[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(pw.p(u));
             }
+          stage_wait<0>();
           __syncthreads();
-          tile_dot<D>(sX, sV, id, dp);  // dP = dO V^T
-          tile_ptx<D>(sP, sX, id, dv);  // dV += P^T dO
+          tile_dot<D>(sDO, sV, id, dp);  // dP = dO V^T
+          tile_ptx<D>(sP, sDO, id, dv);  // dV += P^T dO
           __syncthreads();
-          load_tile<T, D, false>(sX, qg, m0, len, 1.0f);
+          stage_tile<T, D>(sQ, qg, m0, len);
+          stage_commit();
 #pragma unroll
           for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              sP[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(s[i][j] * (dp[i][j] - dl[i]));
+              sDS[(id.ty + 16 * i) * kPPitch + id.tx + 16 * j] = round_to<T>(s[i][j] * (dp[i][j] - dl[i]));
+          stage_wait<0>();
           __syncthreads();
-          tile_ptx<D>(sP, sX, id, dk);  // dK += dS^T Q
+          tile_ptx<D>(sDS, sQ, id, dk);  // dK += dS^T Q
         }
+        m = m2;
       }
+      stage_wait<0>();
     }
   }
   T* dkg = (T*)p.dk + kvoff;
   T* dvg = (T*)p.dv + kvoff;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    int row = n0 + id.ty + 16 * i;
+    const int row = n0 + 4 * id.ty + i;
     if (row >= p.N) continue;
     bool valid = row < len;
 #pragma unroll
     for (int c = 0; c < DC; ++c) {
-      dkg[(size_t)row * D + id.tx + 16 * c] = DT<T>::from_f(valid ? dk[i][c] * p.sm_scale : 0.f);
-      dvg[(size_t)row * D + id.tx + 16 * c] = DT<T>::from_f(valid ? dv[i][c] : 0.f);
+      dkg[(size_t)row * D + Cfg<D>::col(id.tx, c)] = DT<T>::from_f(valid ? dk[i][c] * p.sm_scale : 0.f);
+      dvg[(size_t)row * D + Cfg<D>::col(id.tx, c)] = DT<T>::from_f(valid ? dv[i][c] : 0.f);
     }
   }
 }

@@ -26,9 +26,9 @@ inline int set_smem(K kernel, size_t bytes, const char* what) {
   }
 
 template <typename T> int launch_solve(const Params& p, cudaStream_t st) {
-  dim3 grid(p.nb, p.Hq, p.B);
+  const unsigned grid = (unsigned)((long long)p.nb * p.Hq * p.B);
   ADS_DISPATCH_D(p.D, {
-    size_t sm = 2 * Cfg<DD>::tile_floats * sizeof(float);
+    size_t sm = SolveSmem<DD>::bytes(p.n_words);
     if (int rc = set_smem(solve_kernel<T, DD>, sm, "solve")) return rc;
     solve_kernel<T, DD><<<grid, kThreads, sm, st>>>(p);
   })
@@ -36,9 +36,9 @@ template <typename T> int launch_solve(const Params& p, cudaStream_t st) {
 }
 
 template <typename T> int launch_fwd(const Params& p, cudaStream_t st) {
-  dim3 grid(p.nb, p.Hq, p.B);
+  const unsigned grid = (unsigned)((long long)p.nb * p.Hq * p.B);
   ADS_DISPATCH_D(p.D, {
-    size_t sm = (2 * Cfg<DD>::tile_floats + 2 * 64 * kPPitch) * sizeof(float);
+    size_t sm = ((Cfg<DD>::split ? 3 : 2) * Cfg<DD>::tile_floats + 2 * 64 * kPPitch) * sizeof(float);
     if (int rc = set_smem(fwd_kernel<T, DD>, sm, "fwd")) return rc;
     fwd_kernel<T, DD><<<grid, kThreads, sm, st>>>(p);
   })
@@ -62,15 +62,16 @@ template <typename T> int launch_bwd(const Params& p, cudaStream_t st) {
     if (int rc = check_launch("simt::transpose_bitmap")) return rc;
   }
   ADS_DISPATCH_D(p.D, {
-    size_t sm = (3 * Cfg<DD>::tile_floats + 64 * kPPitch) * sizeof(float);
+    size_t sm = ((Cfg<DD>::split ? 4 : 3) * Cfg<DD>::tile_floats + 64 * kPPitch) * sizeof(float);
     if (stages & ADS_BWD_DQ) {
       if (int rc = set_smem(bwd_dq_kernel<T, DD>, sm, "bwd_dq")) return rc;
-      bwd_dq_kernel<T, DD><<<dim3(p.nb, p.Hq, p.B), kThreads, sm, st>>>(p);
+      bwd_dq_kernel<T, DD><<<(unsigned)((long long)p.nb * p.Hq * p.B), kThreads, sm, st>>>(p);
       if (int rc = check_launch("simt::bwd_dq")) return rc;
     }
     if (stages & ADS_BWD_DKV) {
+      if (Cfg<DD>::split) sm += 64 * kPPitch * sizeof(float);
       if (int rc = set_smem(bwd_dkv_kernel<T, DD>, sm, "bwd_dkv")) return rc;
-      bwd_dkv_kernel<T, DD><<<dim3(p.nb, p.Hkv, p.B), kThreads, sm, st>>>(p);
+      bwd_dkv_kernel<T, DD><<<(unsigned)((long long)p.nb * p.Hkv * p.B), kThreads, sm, st>>>(p);
       if (int rc = check_launch("simt::bwd_dkv")) return rc;
     }
   })

@@ -432,3 +432,30 @@ def test_c_abi_error_codes_on_device():
     sh.path = 9
     rc = lib.adasplash2_fwd(*([q.data_ptr()] * 8), ctypes.byref(sh), None, 0, None, 0, None)
     assert rc == 1 and b"unknown path" in lib.adasplash_last_error_string()
+
+
+@pytest.mark.parametrize("D", [16, 32, 64, 128, 256])
+@pytest.mark.parametrize("scale", [0.05, 1.0, 3.0])
+@pytest.mark.parametrize("N,vl", [(256, [1, 193]), (512, None)])
+def test_fp32_solver_lists_and_sweeps(D, scale, N, vl):
+    # Nearly flat rows overflow the lists (sweeps of S), the others stay on them.  Either way tau solves
+    # sum [z - tau]_+^2 = 1 (fp32 sums of up to N terms below 1: 1e-4 on the sum) and a tile's bit is
+    # set exactly where a score lies above tau, but for scores within the rounding of a score.
+    B, H = 2, 2
+    q, k = _randn((B, H, N, D), 95, scale), _randn((B, H, N, D), 96, 1.0)
+    varlen = None if vl is None else torch.tensor(vl, dtype=torch.int32).cuda()
+    _lib.set_kernel_path("simt")
+    tau, bm = att.solve(q.cuda(), k.cuda(), 10, varlen)
+    z = (0.5 / D ** 0.5) * (q.double() @ k.double().transpose(-1, -2))
+    col, row = torch.arange(N), torch.arange(N)[:, None]
+    for b in range(B):
+        n = N if vl is None else vl[b]
+        zb = z[b].masked_fill((col > row) | (col >= n), float("-inf"))[:, :n]
+        t = tau[b, :, :n, None].cpu().double()
+        assert (((zb - t).clamp(min=0) ** 2).sum(-1) - 1).abs().max() < 1e-4
+        for eps, must in ((1e-4, True), (-1e-4, False)):
+            hit = (zb > t + eps).nonzero()
+            want = torch.zeros((H, N // 64, N // 64), dtype=torch.bool)
+            want[hit[:, 0], hit[:, 1] // 64, hit[:, 2] // 64] = True
+            got = torch.stack([(bm[b, :, :N // 64, j // 32].cpu() >> (j % 32)) & 1 for j in range(N // 64)], -1).bool()
+            assert (got | ~want).all() if must else (want | ~got).all()
