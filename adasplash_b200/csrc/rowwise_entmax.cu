@@ -3,8 +3,8 @@
 // One group of TPR threads owns one row and keeps it in registers, so the row
 // is read from HBM exactly once and the result written once: 8 bytes per fp32
 // element forward, 12 backward.  Reductions are warp shuffles, plus one shared
-// memory hop when a row spans several warps.  Rows too long for registers use a
-// streaming variant that re-reads the row from L2/HBM.
+// memory hop when a row spans several warps.  Longer rows go through one-pass kernels
+// that keep nothing but the row's candidates.
 //
 // Only the elements within 1 of the row maximum can be in the support (the largest
 // probability [z_max - tau]_+^(1/(alpha-1)) is at most 1, so tau >= z_max - 1).  After the
@@ -17,6 +17,8 @@
 // The threshold search follows adasplash/triton_entmax_v2.py:361-536 (4-bin
 // histogram lower bound, quadratic start on the bin-centre model, Halley /
 // Newton / secant / bisection refinement); the backward follows :539-617.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ads {
@@ -47,12 +49,13 @@ struct GroupReduce {
   __device__ GroupReduce(float* s) : smem(s), phase(0) {
     group_warp0 = (threadIdx.x / TPR) * (TPR / 32);
   }
-  template <typename Op>
-  __device__ __forceinline__ void reduce4(float v[4], Op op) {
+  // the first NR of the four values (the others are left as they are)
+  template <int NR = 4, typename Op>
+  __device__ __forceinline__ void reduce(float v[4], Op op) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = op(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
+      for (int i = 0; i < NR; ++i) v[i] = op(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
     }
     if constexpr (TPR > 32) {
       const int warps_cta = blockDim.x / 32;
@@ -60,14 +63,14 @@ struct GroupReduce {
       int w = threadIdx.x / 32;
       if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) buf[w * 4 + i] = v[i];
+        for (int i = 0; i < NR; ++i) buf[w * 4 + i] = v[i];
       }
       group_sync<TPR>();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = buf[group_warp0 * 4 + i];
+      for (int i = 0; i < NR; ++i) v[i] = buf[group_warp0 * 4 + i];
       for (int g = 1; g < TPR / 32; ++g) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = op(v[i], buf[(group_warp0 + g) * 4 + i]);
+        for (int i = 0; i < NR; ++i) v[i] = op(v[i], buf[(group_warp0 + g) * 4 + i]);
       }
       phase ^= 1;
     }
@@ -75,7 +78,6 @@ struct GroupReduce {
 };
 
 struct OpAdd { __device__ __forceinline__ float operator()(float a, float b) const { return a + b; } };
-struct OpMax { __device__ __forceinline__ float operator()(float a, float b) const { return fmaxf(a, b); } };
 
 __device__ __forceinline__ float masked_pow(float x, bool m, float c, int fast_math) {
   // triton_entmax_v2.py:22-39: fast_powf(x, c), or exp2(log2(max(x, 1e-6)) * c) -- both are
@@ -235,6 +237,36 @@ struct RegRow {
       }
     }
   }
+  // Only the chunks of four in which `w` has a non-zero weight (0 elsewhere).  `w` is zero beyond
+  // the row, so such a chunk lies inside it.
+  __device__ __forceinline__ void load_weighted(const T* row, const RegRow& w) {
+    cols = w.cols;
+    tl = w.tl;
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      const float* wc = w.v + c * 4;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[c * 4 + e] = 0.f;
+      if constexpr (VEC) {
+        if (wc[0] != 0.f || wc[1] != 0.f || wc[2] != 0.f || wc[3] != 0.f) {
+          const int c0 = (c * TPR + tl) * 4;
+          if constexpr (sizeof(T) == 4) {
+            const float4 q = *reinterpret_cast<const float4*>(row + c0);
+            v[c * 4 + 0] = q.x; v[c * 4 + 1] = q.y; v[c * 4 + 2] = q.z; v[c * 4 + 3] = q.w;
+          } else {
+            const uint2 q = *reinterpret_cast<const uint2*>(row + c0);
+            const T* h = reinterpret_cast<const T*>(&q);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[c * 4 + e] = DT<T>::to_f(h[e]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (wc[e] != 0.f) v[c * 4 + e] = DT<T>::to_f(row[col_of(c, e)]);
+      }
+    }
+  }
   template <typename F> __device__ __forceinline__ void for_each(F f) const {
 #pragma unroll
     for (int i = 0; i < NV * 4; ++i) f(v[i]);
@@ -289,33 +321,6 @@ struct RegRow {
   }
 };
 
-template <typename T, int TPR>
-struct StreamRow {  // re-reads the row from global memory on every pass
-  const T* row;
-  int cols, tl;
-  float sc;
-  __device__ __forceinline__ void load(const T* r, int cols_, float sc_) {
-    row = r; cols = cols_; sc = sc_; tl = threadIdx.x % TPR;
-  }
-  template <typename F> __device__ __forceinline__ void for_each(F f) const {
-    for (int c = tl; c < cols; c += TPR) f(DT<T>::to_f(row[c]) * sc);
-  }
-  __device__ __forceinline__ float max() const {
-    float m = -INFINITY;
-    for (int c = tl; c < cols; c += TPR) m = fmaxf(m, DT<T>::to_f(row[c]) * sc);
-    return m;
-  }
-  template <typename F> __device__ __forceinline__ void for_each_at_least(float thr, F f) const {
-    for (int c = tl; c < cols; c += TPR) {
-      const float x = DT<T>::to_f(row[c]) * sc;
-      if (x >= thr) f(x);
-    }
-  }
-  template <typename F> __device__ __forceinline__ void store(T* out, F f) const {
-    for (int c = tl; c < cols; c += TPR) out[c] = DT<T>::from_f(f(DT<T>::to_f(row[c]) * sc));
-  }
-};
-
 constexpr int kCandSlots = 8;  // candidates a thread keeps in shared memory (slot j of thread t: [j * blockDim.x + t])
 
 // Maximum over the TPR threads of a row group.  Inside a warp it is one integer reduction on an
@@ -340,6 +345,86 @@ __device__ __forceinline__ float group_max(float x, float* smem_max) {
   return m;
 }
 
+// The threshold search of one row: `each(f)` calls f on every candidate this thread is responsible
+// for and `reduce_sums` adds the partial sums over the threads that take part.  mx: row maximum.
+template <typename Each, typename Reduce>
+__device__ __forceinline__ float entmax_threshold(float mx, float alpha, int mode, int n_iter, int use_hist,
+                                                  int fast_math, Each each, Reduce reduce_sums) {
+  const float c0 = 1.0f / (alpha - 1.0f), c1 = c0 - 1.0f;
+  float red4[4];
+  Hybrid s;
+  if (use_hist && alpha <= 2.0f) {
+    // stage 2: 4-bin histogram of x - (max-1) on [0,1]; cumulative counts
+    // N_b = #{proj*4 >= b} give the same bins as floor(proj*4) clamped to 3.
+    float t_init = mx - 1.0f;
+    float n0 = 0.f, n1 = 0.f, n2 = 0.f, n3 = 0.f;
+    each([&](float x) {
+      const float d = x - t_init;
+      if (d >= 0.f) {  // only the few elements within 1 of the row maximum land in a bin
+        const float p4 = d * (float)kBins;
+        n0 += 1.f;
+        n1 += (p4 >= 1.f) ? 1.f : 0.f;
+        n2 += (p4 >= 2.f) ? 1.f : 0.f;
+        n3 += (p4 >= 3.f) ? 1.f : 0.f;
+      }
+    });
+    red4[0] = n0; red4[1] = n1; red4[2] = n2; red4[3] = n3;
+    reduce_sums(red4, std::integral_constant<int, 4>{});
+    float raw[kBins] = {red4[0] - red4[1], red4[1] - red4[2], red4[2] - red4[3], red4[3]};
+    float t0;
+    if (mode == 0) {
+      int cnt[kBins] = {(int)raw[0], (int)raw[1], (int)raw[2], (int)raw[3]};
+      t0 = hist_tau_alpha15<kBins>(cnt, kBins, t_init);
+    } else {  // alpha == 2 (triton_entmax_v2.py:113-131)
+      float sz = 1.f, sk = 1.f;
+      for (int sj = kBins - 1; sj >= 0; --sj) {
+        float c = raw[sj] - (sj == kBins - 1 ? 1.f : 0.f);
+        float e = (float)sj / kBins;
+        float nz = sz + c * e, nk = sk + c;
+        if ((nz - nk * e) < 1.0f) { sz = nz; sk = nk; }
+      }
+      t0 = t_init + (sz - 1.0f) / sk;
+    }
+    s.lo = t0;
+    s.hi = t0 + 1.0f / kBins;
+    s.t = muller_init(s.lo, s.hi, t_init, raw);
+  } else {
+    s.hi = mx;
+    s.lo = mx - 1.0f;
+    s.t = 0.5f * (s.lo + s.hi);
+  }
+  s.t_prev = s.t;
+  s.f_prev = 0.f;
+  // stage 3: refinement
+  for (int it = 0; it < n_iter; ++it) {
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+    const float t = s.t;
+    if (mode == 1) {
+      each([&](float x) { if (x > t) { a0 += x - t; a1 += 1.f; } });
+    } else if (mode == 0) {
+      each([&](float x) {
+        if (x > t) {  // the support is a small part of the row
+          const float u = x - t;
+          a0 = fmaf(u, u, a0); a1 += u; a2 += 1.f;
+        }
+      });
+    } else {
+      each([&](float x) {
+        if (x > t) {  // the support is a small part of the row: skip the transcendental work elsewhere
+          float p0, p1, p2;
+          pow3(x - t, c0, fast_math, p0, p1, p2);
+          a0 += p0; a1 += p1; a2 += p2;
+        }
+      });
+    }
+    red4[0] = a0; red4[1] = a1; red4[2] = a2;
+    if (mode == 1) reduce_sums(red4, std::integral_constant<int, 2>{});
+    else reduce_sums(red4, std::integral_constant<int, 3>{});
+    hybrid_update(s, red4[0], red4[1], red4[2], c0, c1, alpha, it > 0);
+  }
+  return s.t;
+}
+
 template <typename T, int TPR, typename Row>
 __device__ __forceinline__ void entmax_fwd_row(Row& r, T* yrow, float* tau_out, long long row_idx,
                                                bool row_ok, float alpha, int n_iter, int use_hist,
@@ -347,9 +432,7 @@ __device__ __forceinline__ void entmax_fwd_row(Row& r, T* yrow, float* tau_out, 
                                                float* s_cand) {
   GroupReduce<TPR> red(smem);
   const int mode = (alpha == 1.5f) ? 0 : (alpha == 2.0f ? 1 : 2);
-  const float c0 = 1.0f / (alpha - 1.0f), c1 = c0 - 1.0f, c2 = c1 - 1.0f;
-  (void)c2;
-  float red4[4];
+  const float c0 = 1.0f / (alpha - 1.0f);
   // stage 1: maximum of the scaled row
   const float mx = group_max<TPR>(r.max(), smem_max);
   // Candidates: tau never falls below max - 1 (minus the 1e-6 slack of the bracket test), so
@@ -363,79 +446,6 @@ __device__ __forceinline__ void entmax_fwd_row(Row& r, T* yrow, float* tau_out, 
       ++n_cand;
     });
   }
-  // The threshold search: `each(f)` calls f on every candidate this thread is responsible for and
-  // `reduce_sums` adds the partial sums over the threads that take part.
-  Hybrid s;
-  auto solve = [&](auto each, auto reduce_sums) {
-    if (use_hist && alpha <= 2.0f) {
-      // stage 2: 4-bin histogram of x - (max-1) on [0,1]; cumulative counts
-      // N_b = #{proj*4 >= b} give the same bins as floor(proj*4) clamped to 3.
-      float t_init = mx - 1.0f;
-      float n0 = 0.f, n1 = 0.f, n2 = 0.f, n3 = 0.f;
-      each([&](float x) {
-        const float d = x - t_init;
-        if (d >= 0.f) {  // only the few elements within 1 of the row maximum land in a bin
-          const float p4 = d * (float)kBins;
-          n0 += 1.f;
-          n1 += (p4 >= 1.f) ? 1.f : 0.f;
-          n2 += (p4 >= 2.f) ? 1.f : 0.f;
-          n3 += (p4 >= 3.f) ? 1.f : 0.f;
-        }
-      });
-      red4[0] = n0; red4[1] = n1; red4[2] = n2; red4[3] = n3;
-      reduce_sums(red4);
-      float raw[kBins] = {red4[0] - red4[1], red4[1] - red4[2], red4[2] - red4[3], red4[3]};
-      float t0;
-      if (mode == 0) {
-        int cnt[kBins] = {(int)raw[0], (int)raw[1], (int)raw[2], (int)raw[3]};
-        t0 = hist_tau_alpha15<kBins>(cnt, kBins, t_init);
-      } else {  // alpha == 2 (triton_entmax_v2.py:113-131)
-        float sz = 1.f, sk = 1.f;
-        for (int sj = kBins - 1; sj >= 0; --sj) {
-          float c = raw[sj] - (sj == kBins - 1 ? 1.f : 0.f);
-          float e = (float)sj / kBins;
-          float nz = sz + c * e, nk = sk + c;
-          if ((nz - nk * e) < 1.0f) { sz = nz; sk = nk; }
-        }
-        t0 = t_init + (sz - 1.0f) / sk;
-      }
-      s.lo = t0;
-      s.hi = t0 + 1.0f / kBins;
-      s.t = muller_init(s.lo, s.hi, t_init, raw);
-    } else {
-      s.hi = mx;
-      s.lo = mx - 1.0f;
-      s.t = 0.5f * (s.lo + s.hi);
-    }
-    s.t_prev = s.t;
-    s.f_prev = 0.f;
-    // stage 3: refinement
-    for (int it = 0; it < n_iter; ++it) {
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-      const float t = s.t;
-      if (mode == 1) {
-        each([&](float x) { if (x > t) { a0 += x - t; a1 += 1.f; } });
-      } else if (mode == 0) {
-        each([&](float x) {
-          if (x > t) {  // the support is a small part of the row
-            const float u = x - t;
-            a0 = fmaf(u, u, a0); a1 += u; a2 += 1.f;
-          }
-        });
-      } else {
-        each([&](float x) {
-          if (x > t) {  // the support is a small part of the row: skip the transcendental work elsewhere
-            float p0, p1, p2;
-            pow3(x - t, c0, fast_math, p0, p1, p2);
-            a0 += p0; a1 += p1; a2 += p2;
-          }
-        });
-      }
-      red4[0] = a0; red4[1] = a1; red4[2] = a2; red4[3] = 0.f;
-      reduce_sums(red4);
-      hybrid_update(s, red4[0], red4[1], red4[2], c0, c1, alpha, it > 0);
-    }
-  };
   // Every thread works through its own slots, or through all of its elements if they did not fit
   // (same elements above any threshold >= max - 1 - 1e-5, same order), and the sums are reduced
   // over the group.  Two alternatives were measured slower on 16384 x 4096 (0.117 vs 0.096 ms for
@@ -443,17 +453,18 @@ __device__ __forceinline__ void entmax_fwd_row(Row& r, T* yrow, float* tau_out, 
   // list that every warp works through by itself without barriers, and letting the first warp of
   // the group do the whole search alone.  The search is a dependent chain per row; what pays is
   // more rows in flight, not fewer instructions.
-  solve([&](auto f) {
-          if (n_cand <= kCandSlots) {
-            const float* mine = s_cand + threadIdx.x;
-            for (int j = 0; j < n_cand; ++j) f(mine[j * blockDim.x]);
-          } else {
-            r.for_each(f);
-          }
-        },
-        [&](float v[4]) { red.reduce4(v, OpAdd()); });
+  const float t = entmax_threshold(
+      mx, alpha, mode, n_iter, use_hist, fast_math,
+      [&](auto f) {
+        if (n_cand <= kCandSlots) {
+          const float* mine = s_cand + threadIdx.x;
+          for (int j = 0; j < n_cand; ++j) f(mine[j * blockDim.x]);
+        } else {
+          r.for_each(f);
+        }
+      },
+      [&](float v[4], auto nr) { red.template reduce<decltype(nr)::value>(v, OpAdd()); });
   // stage 4: output
-  const float t = s.t;
   if (row_ok) {
     if (mode == 1) {
       r.store(yrow, [&](float x) { return x > t ? x - t : 0.f; });
@@ -546,19 +557,215 @@ entmax_fwd_pipe_kernel(const T* __restrict__ x, T* __restrict__ y, float* __rest
   }
 }
 
+// ---------------------------------------------------------------------------
+// Rows too long for registers
+// ---------------------------------------------------------------------------
+// One CTA per row, one pass over it.  Bound by HBM: x in and y out once.
+//   * y is zero outside the support, so the pass that reads x also writes a row of zeros, and only
+//     the few candidates are visited again once the threshold is known.
+//   * The candidates are gathered in the same pass, against the largest element the CTA has seen
+//     so far (one shared word, raised by the warps as they go, no barrier): that bound only grows,
+//     so what it lets through is a superset of what the final maximum lets through, and the
+//     threshold search drops the rest.  A thread keeps (value, column) of its own candidates in
+//     its own slots; one with more than fit goes over its elements again (from L2), with the same
+//     terms in the same order, so the result does not depend on how the warps happened to run.
+//   * 16-byte loads on the 16-byte grid of the row's address; the at most 15 elements before
+//     and after that grid go one to a thread.  y has a grid of its own (its base may differ).
+constexpr int kLongBatch = 4;      // 16-byte loads a thread has in flight
+constexpr int kLongSlots = 8;
+// CTAs per SM, one's threshold search (a chain of reductions) beside the others' loads: 1536 threads
+// of fp32 rows, 1024 of 16-bit ones (whose chunks hold twice the elements: they would spill)
+template <typename T> constexpr int long_ctas(int threads) { return (sizeof(T) == 4 ? 1536 : 1024) / threads; }
+
+// The elements of one row as its threads see them: element e < head is thread e's, the body is
+// n_vec chunks of VEC elements dealt round by round, the tail follows it.  `off` is the element
+// offset of the row's first byte from a 16-byte boundary.
+template <int VEC>
+struct LongSplit {
+  int head, n_vec, tail;
+  __device__ __forceinline__ LongSplit(const void* row, int elem_bytes, int cols) {
+    const int off = VEC > 1 ? (int)(((uintptr_t)row & 15) / elem_bytes) : 0;
+    head = min(cols, off ? VEC - off : 0);
+    n_vec = (cols - head) / VEC;
+    tail = cols - head - n_vec * VEC;
+  }
+  __device__ __forceinline__ int tail0() const { return head + n_vec * VEC; }
+};
+
+// VEC elements to fp32 (16 bytes, or a single element when the kernel runs unaligned)
+template <typename T, int VEC> struct Pack { T e[VEC]; };
+template <typename T, int VEC>
+__device__ __forceinline__ Pack<T, VEC> load_pack(const T* p) {
+  Pack<T, VEC> r;
+  if constexpr (VEC > 1) *reinterpret_cast<uint4*>(&r) = *reinterpret_cast<const uint4*>(p);
+  else r.e[0] = *p;
+  return r;
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void store_pack(T* p, const Pack<T, VEC>& v) {
+  if constexpr (VEC > 1) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(&v);
+  else *p = v.e[0];
+}
+
+// f(element index of the first, pack, number of valid elements) over this thread's share, in a
+// fixed order: head, body, tail
+template <typename T, int THREADS, int VEC, typename F>
+__device__ __forceinline__ void long_for_each(const T* row, const LongSplit<VEC>& sp, F f) {
+  const int t = threadIdx.x;
+  if (t < sp.head) f(t, row[t]);
+  for (int i = t; i < sp.n_vec; i += THREADS) {
+    const int c0 = sp.head + i * VEC;
+    const Pack<T, VEC> q = load_pack<T, VEC>(row + c0);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) f(c0 + e, q.e[e]);
+  }
+  if (t < sp.tail) f(sp.tail0() + t, row[sp.tail0() + t]);
+}
+
+// zeros over this thread's share of a row, batch by batch beside the loads
 template <typename T>
-__global__ void __launch_bounds__(1024)
-entmax_fwd_stream_kernel(const T* __restrict__ x, T* __restrict__ y, float* __restrict__ tau_out,
-                         long long rows, int cols, float alpha, int n_iter, int use_hist,
-                         int fast_math) {
+struct LongZero {
+  static constexpr int VEC = 16 / (int)sizeof(T);
+  T* row;
+  LongSplit<VEC> sp;
+  __device__ __forceinline__ LongZero(T* r, int cols) : row(r), sp(r, (int)sizeof(T), cols) {}
+  __device__ __forceinline__ void ends() const {
+    const T z = DT<T>::from_f(0.f);
+    if ((int)threadIdx.x < sp.head) row[threadIdx.x] = z;
+    if ((int)threadIdx.x < sp.tail) row[sp.tail0() + threadIdx.x] = z;
+  }
+  __device__ __forceinline__ void chunk(int i) const {
+    if (i < sp.n_vec) *reinterpret_cast<uint4*>(row + sp.head + i * VEC) = make_uint4(0u, 0u, 0u, 0u);
+  }
+};
+
+// `fill` = 0 (y overlaps x): nothing is written before the threshold is known; every thread then
+// writes all of its elements.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS, long_ctas<T>(THREADS))
+entmax_fwd_long_kernel(const T* x, T* y, float* __restrict__ tau_out, int cols, float alpha, int n_iter,
+                       int use_hist, int fast_math, int fill) {
+  constexpr int VEC = 16 / (int)sizeof(T);
   __shared__ float smem[2 * 32 * 4];
-  __shared__ float smem_max[32];
-  __shared__ float s_cand[kCandSlots * 1024];
-  long long row = blockIdx.x;
-  StreamRow<T, 1024> r;
-  r.load(x + row * cols, cols, alpha - 1.0f);
-  entmax_fwd_row<T, 1024>(r, y + row * cols, tau_out, row, true, alpha, n_iter, use_hist, fast_math, smem,
-                          smem_max, s_cand);
+  __shared__ int s_max;
+  __shared__ float2 s_cand[kLongSlots * THREADS];  // (value, column) of a thread's candidates
+  const long long row_idx = blockIdx.x;
+  const T* xr = x + row_idx * cols;
+  T* yr = y + row_idx * cols;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const float sc = alpha - 1.0f;
+  const LongSplit<VEC> sp(xr, (int)sizeof(T), cols);
+  const LongZero<T> zero(yr, cols);
+  if (tid == 0) s_max = ordered_int(-INFINITY);
+  __syncthreads();
+  float2* mine = s_cand + tid;
+  int n_cand = 0;
+  auto note = [&](float v, int col, float thr) {
+    if (v >= thr) {
+      if (n_cand < kLongSlots) mine[n_cand * THREADS] = make_float2(v, __int_as_float(col));
+      ++n_cand;
+    }
+  };
+  // raises the CTA's maximum and returns the bound it gives
+  auto bound = [&](float m) -> float {
+    const int wm = __reduce_max_sync(0xffffffffu, ordered_int(fmaxf(m, -INFINITY)));  // (a NaN is no maximum)
+    if (lane == 0 && wm > *(volatile int*)&s_max) atomicMax(&s_max, wm);
+    __syncwarp();
+    return ordered_float(max(*(volatile int*)&s_max, wm)) - 1.0f - 1e-5f;
+  };
+  {
+    if (fill) zero.ends();
+    float v = -INFINITY;
+    if (tid < sp.head) v = DT<T>::to_f(xr[tid]) * sc;
+    const float thr = bound(v);
+    if (tid < sp.head) note(v, tid, thr);
+  }
+  const int rounds = max(sp.n_vec, zero.sp.n_vec);
+  for (int base = 0; base < rounds; base += THREADS * kLongBatch) {
+    Pack<T, VEC> q[kLongBatch];
+#pragma unroll
+    for (int j = 0; j < kLongBatch; ++j) {
+      const int i = base + j * THREADS + tid;
+      if (i < sp.n_vec) q[j] = load_pack<T, VEC>(xr + sp.head + i * VEC);
+      else {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) q[j].e[e] = DT<T>::from_f(-INFINITY);
+      }
+    }
+    if (fill) {
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j) zero.chunk(base + j * THREADS + tid);
+    }
+    float mj[kLongBatch], m = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kLongBatch; ++j) {
+      mj[j] = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) mj[j] = fmaxf(mj[j], DT<T>::to_f(q[j].e[e]) * sc);
+      m = fmaxf(m, mj[j]);
+    }
+    const float thr = bound(m);
+    if (m >= thr) {
+#pragma unroll
+      for (int j = 0; j < kLongBatch; ++j) {
+        const int i = base + j * THREADS + tid;
+        if (mj[j] >= thr && i < sp.n_vec) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) note(DT<T>::to_f(q[j].e[e]) * sc, sp.head + i * VEC + e, thr);
+        }
+      }
+    }
+  }
+  {
+    float v = -INFINITY;
+    if (tid < sp.tail) v = DT<T>::to_f(xr[sp.tail0() + tid]) * sc;
+    const float thr = bound(v);
+    if (tid < sp.tail) note(v, sp.tail0() + tid, thr);
+  }
+  __syncthreads();  // the maximum is final, and the zeros of every thread are written
+  const float mx = ordered_float(s_max);
+  const int mode = (alpha == 1.5f) ? 0 : (alpha == 2.0f ? 1 : 2);
+  const float c0 = 1.0f / (alpha - 1.0f);
+  const float thr = mx - 1.0f - 1e-5f;
+  GroupReduce<THREADS> red(smem);
+  const bool listed = n_cand <= kLongSlots;
+  const float t = entmax_threshold(
+      mx, alpha, mode, n_iter, use_hist, fast_math,
+      [&](auto f) {
+        if (listed) {
+          for (int j = 0; j < n_cand; ++j) {
+            const float v = mine[j * THREADS].x;
+            if (v >= thr) f(v);
+          }
+        } else {
+          long_for_each<T, THREADS, VEC>(xr, sp, [&](int, T e) {
+            const float v = DT<T>::to_f(e) * sc;
+            if (v >= thr) f(v);
+          });
+        }
+      },
+      [&](float v[4], auto nr) { red.template reduce<decltype(nr)::value>(v, OpAdd()); });
+  auto value = [&](float v) -> T {
+    float o;
+    if (mode == 1) o = v > t ? v - t : 0.f;
+    else if (mode == 0) { const float u = v > t ? v - t : 0.f; o = u * u; }
+    else o = masked_pow(fmaxf(v - t, 0.f), v > t, c0, fast_math);
+    return DT<T>::from_f(o);
+  };
+  if (!fill) {
+    long_for_each<T, THREADS, VEC>(xr, sp, [&](int col, T e) { yr[col] = value(DT<T>::to_f(e) * sc); });
+  } else if (listed) {
+    for (int j = 0; j < n_cand; ++j) {
+      const float2 c = mine[j * THREADS];
+      if (c.x > t) yr[__float_as_int(c.y)] = value(c.x);
+    }
+  } else {
+    long_for_each<T, THREADS, VEC>(xr, sp, [&](int col, T e) {
+      const float v = DT<T>::to_f(e) * sc;
+      if (v > t) yr[col] = value(v);
+    });
+  }
+  if (tau_out != nullptr && tid == 0) tau_out[row_idx] = t;
 }
 
 // ---------------------------------------------------------------------------
@@ -571,7 +778,7 @@ __device__ __forceinline__ float bwd_u(float y, float alpha, int mode, int fast_
   return masked_pow(y, m, 2.0f - alpha, fast_math);
 }
 
-template <typename T, int TPR, int NV, bool VEC>
+template <typename T, int TPR, int NV, bool VEC, bool SKIP>
 __global__ void __launch_bounds__((TPR > 128 ? TPR : 128))
 entmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx,
                       long long rows, int cols, float alpha, int fast_math) {
@@ -582,22 +789,28 @@ entmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __re
   long long rr = ok ? row : rows - 1;
   const int mode = (alpha == 1.5f) ? 0 : (alpha == 2.0f ? 1 : 2);
   RegRow<T, TPR, NV, VEC> ry, rdy;
+  // The weights of an entmax row are zero outside its support, and dy counts only where they are
+  // not.  SKIP: it is fetched for those chunks alone, which for sparse rows is a sector here and there
+  // instead of a third of the kernel's traffic, at the price of a second round trip per row.
+  // 16384 x 4096 fp32: 125 -> 98 us; 65536 x 1000 bf16: 139 -> 188 us, hence for long rows only.
+  // (Slots beyond the row hold y = -inf: weight 0.)
   ry.load(y + rr * cols, cols, 1.0f);
-  rdy.load(dy + rr * cols, cols, 1.0f);
+  if constexpr (!SKIP) rdy.load(dy + rr * cols, cols, 1.0f);
+#pragma unroll
+  for (int i = 0; i < NV * 4; ++i) ry.v[i] = bwd_u(ry.v[i], alpha, mode, fast_math);
+  if constexpr (SKIP) rdy.load_weighted(dy + rr * cols, ry);
   float su = 0.f, sud = 0.f;
 #pragma unroll
   for (int i = 0; i < NV * 4; ++i) {
-    // out-of-range slots hold -inf in both rows: y > 0 is false there, u = 0
-    float u = bwd_u(ry.v[i], alpha, mode, fast_math);
-    ry.v[i] = u;
-    float d = (u != 0.f) ? rdy.v[i] : 0.f;
+    const float u = ry.v[i];
+    const float d = (u != 0.f) ? rdy.v[i] : 0.f;
     rdy.v[i] = d;
     su += u;
     sud = fmaf(u, d, sud);
   }
   GroupReduce<TPR> red(smem);
   float red4[4] = {su, sud, 0.f, 0.f};
-  red.reduce4(red4, OpAdd());
+  red.template reduce<2>(red4, OpAdd());
   float scalar = red4[1] / red4[0];
   if (ok) {
     // grad = u*dy - scalar*u (triton_entmax_v2.py:616)
@@ -607,31 +820,106 @@ entmax_bwd_reg_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __re
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(1024)
-entmax_bwd_stream_kernel(const T* __restrict__ y, const T* __restrict__ dy, T* __restrict__ dx,
-                         long long rows, int cols, float alpha, int fast_math) {
+// Backward of such rows, in the same manner: y is read once, dx is written as zeros beside that, and
+// the columns of the support wait in each thread's slots for the row's scalar.  dy is fetched for the
+// chunks with a non-zero weight alone, or (ALL) in full: it then enters the sum with its weight, zero
+// or not, so that an infinity or NaN anywhere in dy makes the scalar non-finite, and the row is
+// computed element by element.  VEC = 1 when y and dy do not share their offset from a 16-byte boundary.
+template <typename T, int THREADS, int VEC, bool ALL>
+__global__ void __launch_bounds__(THREADS, long_ctas<T>(THREADS))
+entmax_bwd_long_kernel(const T* y, const T* dy, T* dx, int cols, float alpha, int fast_math, int fill) {
   __shared__ float smem[2 * 32 * 4];
-  long long row = blockIdx.x;
+  __shared__ int s_col[kLongSlots * THREADS];
+  const long long row = blockIdx.x;
   const int mode = (alpha == 1.5f) ? 0 : (alpha == 2.0f ? 1 : 2);
   const T* yr = y + row * cols;
   const T* dr = dy + row * cols;
-  float su = 0.f, sud = 0.f;
-  for (int c = threadIdx.x; c < cols; c += 1024) {
-    float u = bwd_u(DT<T>::to_f(yr[c]), alpha, mode, fast_math);
-    su += u;
-    sud = fmaf(u, DT<T>::to_f(dr[c]), sud);
-  }
-  GroupReduce<1024> red(smem);
-  float red4[4] = {su, sud, 0.f, 0.f};
-  red.reduce4(red4, OpAdd());
-  float scalar = red4[1] / red4[0];
   T* xr = dx + row * cols;
-  for (int c = threadIdx.x; c < cols; c += 1024) {
-    float u = bwd_u(DT<T>::to_f(yr[c]), alpha, mode, fast_math);
-    xr[c] = DT<T>::from_f(u * DT<T>::to_f(dr[c]) - scalar * u);
+  const int tid = threadIdx.x;
+  const LongSplit<VEC> sp(yr, (int)sizeof(T), cols);
+  const LongZero<T> zero(xr, cols);
+  int* mine = s_col + tid;
+  int n_sup = 0;
+  float su = 0.f, sud = 0.f;
+  auto add = [&](T ye, T de, int col) {
+    const float u = bwd_u(DT<T>::to_f(ye), alpha, mode, fast_math);
+    su += u;
+    if (ALL) sud = fmaf(u, DT<T>::to_f(de), sud);
+    if (u != 0.f) {
+      if (!ALL) sud = fmaf(u, DT<T>::to_f(de), sud);
+      if (n_sup < kLongSlots) mine[n_sup * THREADS] = col;
+      ++n_sup;
+    }
+  };
+  if (fill) zero.ends();
+  if (tid < sp.head) add(yr[tid], dr[tid], tid);
+  constexpr int BATCH = ALL && VEC > 1 ? kLongBatch / 2 : kLongBatch;
+  const int rounds = max(sp.n_vec, zero.sp.n_vec);
+  for (int base = 0; base < rounds; base += THREADS * BATCH) {
+    Pack<T, VEC> qy[BATCH], qd[BATCH];
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      const int i = base + j * THREADS + tid;
+      if (i < sp.n_vec) {
+        qy[j] = load_pack<T, VEC>(yr + sp.head + i * VEC);
+        if (ALL) qd[j] = load_pack<T, VEC>(dr + sp.head + i * VEC);
+      }
+    }
+    if (fill) {
+#pragma unroll
+      for (int j = 0; j < BATCH; ++j) zero.chunk(base + j * THREADS + tid);
+    }
+    bool on[BATCH];
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      const int i = base + j * THREADS + tid;
+      on[j] = ALL && i < sp.n_vec;
+      if (!ALL && i < sp.n_vec) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) on[j] = on[j] || DT<T>::to_f(qy[j].e[e]) > 0.f;
+        if (on[j]) qd[j] = load_pack<T, VEC>(dr + sp.head + i * VEC);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      const int i = base + j * THREADS + tid;
+      if (on[j]) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) add(qy[j].e[e], qd[j].e[e], sp.head + i * VEC + e);
+      }
+    }
+  }
+  if (tid < sp.tail) add(yr[sp.tail0() + tid], dr[sp.tail0() + tid], sp.tail0() + tid);
+  GroupReduce<THREADS> red(smem);
+  float red4[4] = {su, sud, 0.f, 0.f};
+  red.template reduce<2>(red4, OpAdd());  // (its barrier also orders the zeros before what follows)
+  const float scalar = red4[1] / red4[0];
+  auto grad = [&](int col, T ye) {
+    const float u = bwd_u(DT<T>::to_f(ye), alpha, mode, fast_math);
+    const float d = ALL || u != 0.f ? DT<T>::to_f(dr[col]) : 0.f;
+    xr[col] = DT<T>::from_f(u * d - scalar * u);
+  };
+  if (fill && n_sup <= kLongSlots && fabsf(scalar) < INFINITY) {
+    for (int j = 0; j < n_sup; ++j) {
+      const int col = mine[j * THREADS];
+      grad(col, yr[col]);
+    }
+  } else {
+    long_for_each<T, THREADS, VEC>(yr, sp, [&](int col, T ye) { grad(col, ye); });
   }
 }
+
+// whether [a, a + n) and [b, b + n) share a byte
+inline bool overlap(const void* a, const void* b, size_t n) {
+  const uintptr_t ua = (uintptr_t)a, ub = (uintptr_t)b;
+  return ua < ub + n && ub < ua + n;
+}
+
+// Rows beyond these lengths take the one-pass kernels.  Measured, forward / backward in us, register or
+// old streaming kernel against one pass: 2048 x 50001 fp32 303 / 536 -> 154 / 201; 4096 x 20000 321 / 325 ->
+// 145 / 158; 8192 x 10000 324 / 215 -> 132 / 125; 16384 x 5001 (unaligned) 656 / 174 -> 124 / 122; but 16384 x
+// 4096 98 / 96 -> 108 / 100, and 65536 x 1001 133 / 119 -> 338 / 176: shorter rows stay in registers.
+constexpr int64_t kLongFrom = 4096, kLongFromUnaligned = 2048;
 
 template <typename T, int TPR, int NV>
 int launch_fwd_cfg(const T* x, T* y, float* tau, long long rows, int cols, float alpha, int n_iter,
@@ -663,29 +951,34 @@ int launch_fwd(const void* xv, void* yv, float* tau, long long rows, long long c
   bool vec = (cols % 4 == 0) && ((uintptr_t)x % vec_bytes == 0) && ((uintptr_t)y % vec_bytes == 0);
   int c = (int)cols;
 #define ADS_FWD(TPR, NV) return launch_fwd_cfg<T, TPR, NV>(x, y, tau, rows, c, alpha, n_iter, use_hist, fast_math, vec, st)
-  if (cols <= 128) ADS_FWD(32, 1);
-  if (cols <= 512) ADS_FWD(32, 4);
-  if (cols <= 1024) ADS_FWD(32, 8);
-  if (cols <= 2048) ADS_FWD(64, 8);
-  if (cols <= 4096) ADS_FWD(128, 8);  // measured best of (32,32), (64,16), (128,8), (256,4) on 16384 x 4096
-  if (cols <= 8192) ADS_FWD(256, 8);
-  if (cols <= 16384) ADS_FWD(512, 8);
-  if (cols <= 32768) ADS_FWD(1024, 8);
+  if (vec || cols <= kLongFromUnaligned) {
+    if (cols <= 128) ADS_FWD(32, 1);
+    if (cols <= 512) ADS_FWD(32, 4);
+    if (cols <= 1024) ADS_FWD(32, 8);
+    if (cols <= 2048) ADS_FWD(64, 8);
+    if (cols <= kLongFrom) ADS_FWD(128, 8);  // measured best of (32,32), (64,16), (128,8), (256,4) on 16384 x 4096
+  }
 #undef ADS_FWD
-  entmax_fwd_stream_kernel<T><<<(unsigned)rows, 1024, 0, st>>>(x, y, tau, rows, c, alpha, n_iter, use_hist, fast_math);
-  return check_launch("entmax_fwd_stream");
+  const int fill = !overlap(x, y, (size_t)rows * cols * sizeof(T));
+#define ADS_FWD_LONG(THREADS) \
+  entmax_fwd_long_kernel<T, THREADS><<<(unsigned)rows, THREADS, 0, st>>>(x, y, tau, c, alpha, n_iter, use_hist, fast_math, fill)
+  if (cols <= 8192) ADS_FWD_LONG(128);
+  else if (cols <= 16384) ADS_FWD_LONG(256);
+  else ADS_FWD_LONG(512);
+#undef ADS_FWD_LONG
+  return check_launch("entmax_fwd_long");
 }
 
-template <typename T, int TPR, int NV>
+template <typename T, int TPR, int NV, bool SKIP>
 int launch_bwd_cfg(const T* y, const T* dy, T* dx, long long rows, int cols, float alpha,
                    int fast_math, bool vec, cudaStream_t st) {
   const int threads = TPR > 128 ? TPR : 128;
   const int rpc = threads / TPR;
   unsigned grid = (unsigned)((rows + rpc - 1) / rpc);
   if (vec)
-    entmax_bwd_reg_kernel<T, TPR, NV, true><<<grid, threads, 0, st>>>(y, dy, dx, rows, cols, alpha, fast_math);
+    entmax_bwd_reg_kernel<T, TPR, NV, true, SKIP><<<grid, threads, 0, st>>>(y, dy, dx, rows, cols, alpha, fast_math);
   else
-    entmax_bwd_reg_kernel<T, TPR, NV, false><<<grid, threads, 0, st>>>(y, dy, dx, rows, cols, alpha, fast_math);
+    entmax_bwd_reg_kernel<T, TPR, NV, false, SKIP><<<grid, threads, 0, st>>>(y, dy, dx, rows, cols, alpha, fast_math);
   return check_launch("entmax_bwd");
 }
 
@@ -698,17 +991,29 @@ int launch_bwd(const void* yv, const void* dyv, void* dxv, long long rows, long 
   const size_t vb = 4 * sizeof(T);
   bool vec = (cols % 4 == 0) && ((uintptr_t)y % vb == 0) && ((uintptr_t)dy % vb == 0) && ((uintptr_t)dx % vb == 0);
   int c = (int)cols;
-#define ADS_BWD(TPR, NV) return launch_bwd_cfg<T, TPR, NV>(y, dy, dx, rows, c, alpha, fast_math, vec, st)
-  if (cols <= 128) ADS_BWD(32, 1);
-  if (cols <= 512) ADS_BWD(32, 4);
-  if (cols <= 1024) ADS_BWD(64, 4);
-  if (cols <= 2048) ADS_BWD(128, 4);
-  if (cols <= 4096) ADS_BWD(256, 4);
-  if (cols <= 8192) ADS_BWD(512, 4);
-  if (cols <= 16384) ADS_BWD(1024, 4);
+#define ADS_BWD(TPR, NV, SKIP) return launch_bwd_cfg<T, TPR, NV, SKIP>(y, dy, dx, rows, c, alpha, fast_math, vec, st)
+  if (vec || cols <= kLongFromUnaligned) {
+    if (cols <= 128) ADS_BWD(32, 1, false);
+    if (cols <= 512) ADS_BWD(32, 4, false);
+    if (cols <= 1024) ADS_BWD(128, 2, false);  // 65536 x 1000 bf16: 90 us, (32, 8) 108, (64, 4) 137
+    if (cols <= 2048) ADS_BWD(128, 4, false);
+    if (cols <= kLongFrom) ADS_BWD(256, 4, true);
+  }
 #undef ADS_BWD
-  entmax_bwd_stream_kernel<T><<<(unsigned)rows, 1024, 0, st>>>(y, dy, dx, rows, c, alpha, fast_math);
-  return check_launch("entmax_bwd_stream");
+  const size_t nbytes = (size_t)rows * cols * sizeof(T);
+  const int fill = !overlap(y, dx, nbytes) && !overlap(dy, dx, nbytes);
+  constexpr int VEC = 16 / (int)sizeof(T);
+  const bool same = (((uintptr_t)y ^ (uintptr_t)dy) & 15) == 0;
+#define ADS_BWD_LONG(THREADS, ALL)                                                                                        \
+  do {                                                                                                                    \
+    if (same) entmax_bwd_long_kernel<T, THREADS, VEC, ALL><<<(unsigned)rows, THREADS, 0, st>>>(y, dy, dx, c, alpha, fast_math, fill); \
+    else entmax_bwd_long_kernel<T, THREADS, 1, ALL><<<(unsigned)rows, THREADS, 0, st>>>(y, dy, dx, c, alpha, fast_math, fill);       \
+  } while (0)
+  if (cols <= 8192) ADS_BWD_LONG(128, false);
+  else if (cols <= 16384) ADS_BWD_LONG(256, false);
+  else ADS_BWD_LONG(512, true);
+#undef ADS_BWD_LONG
+  return check_launch("entmax_bwd_long");
 }
 
 }  // namespace

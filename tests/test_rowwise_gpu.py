@@ -186,3 +186,63 @@ def test_many_rows_take_the_pipelined_kernel(rows, cols, dtype, alpha):
     # inputs, so the row sums are only near 1)
     sums = y.float().sum(-1)
     assert sums.min() > 0.8 and sums.max() < 1.2
+
+
+@pytest.mark.parametrize("cols", [16385, 32769, 40003, 50001])   # first lengths past the register kernels, odd ones
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("alpha", [1.333, 1.5, 2.0])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_rows_longer_than_registers(cols, dtype, alpha, offset):
+    # Rows start anywhere in a 16-byte chunk, y (allocated by the call) and dy (offset) do not share
+    # their alignment; flat rows (more candidates than a thread keeps) beside peaked ones.
+    def at_offset(t):
+        buf = torch.zeros(t.numel() + offset, dtype=t.dtype, device="cuda")
+        buf[offset:] = t.flatten().cuda()
+        return buf[offset:].view(t.shape)
+    x = torch.cat([_randn((2, cols), 41, 4.0), _randn((2, cols), 42, 0.2)]).to(dtype)
+    dy = _randn((4, cols), 43, 1.0, dtype)
+    xc = at_offset(x).requires_grad_(True)
+    y = adasplash.triton_entmax(xc, alpha=alpha, n_iter=10)
+    (dx,) = torch.autograd.grad(y, xc, at_offset(dy))
+    p, _ = O.entmax_bisect_exact(x.float(), alpha)
+    assert (y.float().cpu().double() - p).abs().max() < _fwd_tol(dtype, alpha)
+    dxe = O.entmax_backward_exact(y.float().cpu(), dy.float(), alpha)
+    assert (dx.float().cpu().double() - dxe).abs().max() < (1e-2 if dtype == torch.float32 else 5e-2)
+
+
+@pytest.mark.parametrize("cols", [40003])
+def test_long_rows_in_place_and_with_special_values(cols):
+    lib = em._lib.load()
+    st = torch.cuda.current_stream().cuda_stream
+    x = _randn((3, cols), 44, 3.0)
+    x[1, 5:] = float("-inf")          # a support of a few columns
+    x[2, 7] = float("nan")            # never in the support
+    a = x.cuda()
+    y = adasplash.triton_entmax(a, alpha=1.5)
+    assert (y[1, 5:] == 0).all() and y[2, 7] == 0 and torch.isfinite(y).all()
+    assert (y.sum(-1) - 1).abs().max() < 1e-2
+    b = a.clone()                     # the C entry point on one buffer
+    assert lib.adasplash_entmax_fwd(b.data_ptr(), b.data_ptr(), None, 3, cols, 1.5, 2, 1, 0, 0, st) == 0
+    assert torch.equal(b, y)
+    dy = _randn((3, cols), 45).cuda()
+    dx = torch.empty_like(y)
+    assert lib.adasplash_entmax_bwd(y.data_ptr(), dy.data_ptr(), dx.data_ptr(), 3, cols, 1.5, 0, 0, st) == 0
+    c = dy.clone()
+    assert lib.adasplash_entmax_bwd(y.data_ptr(), c.data_ptr(), c.data_ptr(), 3, cols, 1.5, 0, 0, st) == 0
+    assert torch.equal(c, dx)
+    dy[0, int((y[0] == 0).nonzero()[0])] = float("inf")   # counts, weight 0 or not: 0 * inf
+    (dx2,) = (torch.empty_like(y),)
+    assert lib.adasplash_entmax_bwd(y.data_ptr(), dy.data_ptr(), dx2.data_ptr(), 3, cols, 1.5, 0, 0, st) == 0
+    assert dx2[0].isnan().any() and torch.equal(dx2[1:], dx[1:])
+
+
+@pytest.mark.parametrize("shape", [(3, 127), (5, 1000), (3, 4096), (2, 16384), (3, 4095)])
+@pytest.mark.parametrize("alpha", [1.333, 1.5, 2.0])
+def test_backward_reads_dy_on_the_support_only(shape, alpha):
+    # rows that fit registers ignore dy where the weight is zero, whatever it holds
+    x = _randn(shape, 46, 3.0).cuda().requires_grad_(True)
+    y = adasplash.triton_entmax(x, alpha=alpha, n_iter=10)
+    dy = _randn(shape, 47).cuda()
+    (a,) = torch.autograd.grad(y, x, dy, retain_graph=True)
+    (b,) = torch.autograd.grad(y, x, torch.where(y > 0, dy, torch.full_like(dy, float("nan"))))
+    assert torch.equal(a, b)
