@@ -137,7 +137,10 @@ struct Hybrid {
   float t, lo, hi, t_prev, f_prev;
 };
 
-__device__ __forceinline__ void hybrid_update(Hybrid& s, float a0, float a1, float a2, float c0,
+// Returns whether the step is a fixed point: a Halley or Newton step that lands on the t it started
+// from, inside a bracket that already takes this t's sign into account.  (A secant or bisection
+// step depends on more than t and is never one.)
+__device__ __forceinline__ bool hybrid_update(Hybrid& s, float a0, float a1, float a2, float c0,
                                               float c1, float alpha, bool allow_secant) {
   // triton_entmax_v2.py:42-110
   const float eps = 1e-6f, eps_den = 1e-12f;
@@ -160,6 +163,7 @@ __device__ __forceinline__ void hybrid_update(Hybrid& s, float a0, float a1, flo
               (alpha <= 2.0f);
     if (ok) { cand = tn; has = true; }
   }
+  const bool fixed = has && cand == t;
   if (!has && allow_secant) {
     float den = ff - s.f_prev;
     float ts = t - ff * (t - s.t_prev) / den;
@@ -169,6 +173,7 @@ __device__ __forceinline__ void hybrid_update(Hybrid& s, float a0, float a1, flo
   s.t_prev = t;
   s.f_prev = ff;
   s.t = has ? cand : 0.5f * (s.lo + s.hi);
+  return fixed;
 }
 
 // ---------------------------------------------------------------------------
@@ -420,7 +425,9 @@ __device__ __forceinline__ float entmax_threshold(float mx, float alpha, int mod
     red4[0] = a0; red4[1] = a1; red4[2] = a2;
     if (mode == 1) reduce_sums(red4, std::integral_constant<int, 2>{});
     else reduce_sums(red4, std::integral_constant<int, 3>{});
-    hybrid_update(s, red4[0], red4[1], red4[2], c0, c1, alpha, it > 0);
+    // The steps that are left from a fixed point would sum the same terms and stay there: the
+    // result is that of all n_iter steps, bit for bit (and every thread of the row sees the same sums).
+    if (hybrid_update(s, red4[0], red4[1], red4[2], c0, c1, alpha, it > 0)) break;
   }
   return s.t;
 }
