@@ -162,28 +162,52 @@ __global__ void __launch_bounds__(kRowThreads) fwd_rows_kernel(RowsParams p) {
 }
 
 // Largest squared norm of a key row per kv head (the solver's export needs it above alpha = 1.5
-// to bound the difference between the two roundings of a score).  One warp per key row.
-template <typename T>
+// to bound the difference between the two roundings of a score).  Reads K once, 16 bytes per lane
+// with D/8 lanes on a row, and ends with one atomic per CTA of kNormRows rows.  Bound by HBM (or L2,
+// where the solver finds K again).
+constexpr int kNormRows = 512;
+
+template <typename T, int D>
 __global__ void __launch_bounds__(256) key_norm_max_kernel(const T* __restrict__ k, float* __restrict__ kmax2,
-                                                           const void* varlen, int is_i64, int B, int Hkv, int N, int D) {
-  const long long row_g = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row_g >= (long long)B * Hkv * N) return;
-  const int lane = threadIdx.x & 31;
-  const int bkv = (int)(row_g / N), r = (int)(row_g % N);
-  if (r >= load_len(varlen, is_i64, bkv / Hkv, N)) return;
-  float s = 0.f;
-  for (int d = lane; d < D; d += 32) { const float x = DT<T>::to_f(k[row_g * D + d]); s = fmaf(x, x, s); }
+                                                           const void* varlen, int is_i64, int Hkv, int N) {
+  constexpr int LPR = D / 8, ROWS = 256 / LPR;  // lanes per row, rows per pass
+  __shared__ int s_max[8];
+  const int per_head = (N + kNormRows - 1) / kNormRows;
+  const int bkv = blockIdx.x / per_head, r0 = (blockIdx.x % per_head) * kNormRows;
+  const int end = min(r0 + kNormRows, load_len(varlen, is_i64, bkv / Hkv, N));
+  if (r0 >= end) return;
+  const int sub = threadIdx.x / LPR, li = threadIdx.x % LPR;
+  const T* kh = k + (size_t)bkv * N * D + li * 8;
+  int m = 0;  // non-negative floats order as ints
+#pragma unroll 4
+  for (int r = r0 + sub; r < r0 + kNormRows; r += ROWS) {
+    float2 f[4];
+    const bool in = r < end;
+    unpack8<T>(in ? *reinterpret_cast<const uint4*>(kh + (size_t)r * D) : make_uint4(0u, 0u, 0u, 0u), f);
+    float2 s2 = splat(0.f);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) atomicMax(reinterpret_cast<int*>(kmax2) + bkv, __float_as_int(s));  // non-negative floats order as ints
+    for (int e = 0; e < 4; ++e) s2 = __ffma2_rn(f[e], f[e], s2);
+    float s = s2.x + s2.y;
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    m = max(m, __float_as_int(s));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = max(m, s_max[w]);
+    atomicMax(reinterpret_cast<int*>(kmax2) + bkv, m);
+  }
 }
 
 template <typename T>
 int key_norms_t(const simt::Params& p, cudaStream_t st) {
   const sup::View sv = sup::view(p.support, nullptr, p.B, p.Hq, p.Hkv, p.N);
-  const long long rows = (long long)p.B * p.Hkv * p.N;
-  key_norm_max_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const T*)p.k, sv.kmax2, p.varlen, p.varlen_is_i64,
-                                                                   p.B, p.Hkv, p.N, p.D);
+  const unsigned grid = (unsigned)((long long)p.B * p.Hkv * ((p.N + kNormRows - 1) / kNormRows));
+  auto kernel = p.D > 64 ? key_norm_max_kernel<T, 128> : key_norm_max_kernel<T, 64>;
+  kernel<<<grid, 256, 0, st>>>((const T*)p.k, sv.kmax2, p.varlen, p.varlen_is_i64, p.Hkv, p.N);
   return check_launch("sparse::key_norm_max");
 }
 
