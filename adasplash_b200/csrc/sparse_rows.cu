@@ -57,38 +57,44 @@ __device__ __forceinline__ uint4 pack8(const float2* f) {
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
 
 // The four row groups of a warp work in lockstep on one row each, as long as the longest of the
-// four supports; so each group takes its eight rows in the order of their entry counts, and rows
+// four supports; so each group takes its RPG rows in the order of their entry counts, and rows
 // of similar length meet.  Returns this lane's row's rank inside its group (0 = most entries).
+template <int RPG>
 __device__ __forceinline__ int rank_in_group(uint32_t cnt, int lane) {
   int rank = 0;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint32_t cj = __shfl_sync(0xffffffffu, cnt, (lane & ~7) + j);
-    rank += (cj > cnt || (cj == cnt && j < (lane & 7))) ? 1 : 0;
+  for (int j = 0; j < RPG; ++j) {
+    const uint32_t cj = __shfl_sync(0xffffffffu, cnt, (lane & ~(RPG - 1)) + j);
+    rank += (cj > cnt || (cj == cnt && j < (lane & (RPG - 1)))) ? 1 : 0;
   }
   return rank;
 }
-// The row (0..31) of group `grp` whose rank is `i`.
+// The row (0 .. 4 RPG - 1) of group `grp` whose rank is `i`.
+template <int RPG>
 __device__ __forceinline__ int row_of_rank(int my_rank, int i, int grp) {
   const uint32_t sel = __ballot_sync(0xffffffffu, my_rank == i);
-  return grp * 8 + __ffs((sel >> (grp * 8)) & 0xffu) - 1;
+  return grp * RPG + __ffs((sel >> (grp * RPG)) & ((1u << RPG) - 1u)) - 1;
 }
 
 // One warp per 32 consecutive query rows of a head, eight lanes per row: lane gl of a group owns
 // the 16-byte chunks gl and (CH = 2, head dim 128) 8 + gl of the head dimension, so a V row is
 // one or two coalesced 128-byte requests per group and every instruction of the accumulation
-// serves four (row, key) pairs.  Group g takes rows 8g .. 8g+7 one after the other; the eight
+// serves four (row, key) pairs.  Group g takes RPG rows one after the other; the eight
 // lanes fetch up to eight of the row's entries with one load and pass them round with shuffles.
-constexpr int kRowsPerWarp = 32;
+// RPG = 8 lets rows of similar length meet; RPG = 2 is for problems whose warps would otherwise
+// leave the chip idle (a row is a chain of dependent loads, and eight of them in turn are what a
+// small problem then takes).
+constexpr int kRowsPerWarp = 32;   // of the backward, and of the forward at RPG = 8
 
-template <typename T, int CH>
+template <typename T, int CH, int RPG>
 __global__ void __launch_bounds__(kRowThreads) fwd_rows_kernel(RowsParams p) {
+  constexpr int kRows = 4 * RPG;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane >> 3, gl = lane & 7;
-  const int chunks = (p.N + kRowsPerWarp - 1) / kRowsPerWarp;  // per head
+  const int chunks = (p.N + kRows - 1) / kRows;  // per head
   const long long wg = (long long)blockIdx.x * (kRowThreads / 32) + warp;
   if (wg >= (long long)p.B * p.Hq * chunks) return;
-  const int bh = (int)(wg / chunks), r0 = (int)(wg % chunks) * kRowsPerWarp;
+  const int bh = (int)(wg / chunks), r0 = (int)(wg % chunks) * kRows;
   const int b = bh / p.Hq, h = bh % p.Hq;
   const int kvh = h / (p.Hq / p.Hkv);
   if (p.sv.dense[b * p.Hkv + kvh] != 0) return;  // the tile kernels own this head
@@ -96,13 +102,13 @@ __global__ void __launch_bounds__(kRowThreads) fwd_rows_kernel(RowsParams p) {
   const int len = load_len(p.varlen, p.varlen_is_i64, b, p.N);
   const size_t row_base = (size_t)bh * p.N;
   // rows at or beyond the sequence length have no entries (the solver wrote nothing for them)
-  const uint2 rw = (r0 + lane < len) ? p.sv.rows[row_base + r0 + lane] : make_uint2(0u, 0u);
+  const uint2 rw = (lane < kRows && r0 + lane < len) ? p.sv.rows[row_base + r0 + lane] : make_uint2(0u, 0u);
   const T* vb = (const T*)p.v + (size_t)(b * p.Hkv + kvh) * p.N * p.Dg + gl * 8;
   const simt::Powers powers(p.alpha);
-  const int my_rank = rank_in_group(rw.y, lane);
+  const int my_rank = rank_in_group<RPG>(rw.y, lane);
 #pragma unroll 1
-  for (int i = 0; i < 8; ++i) {
-    const int rr = row_of_rank(my_rank, i, grp);  // this group's row inside the chunk
+  for (int i = 0; i < RPG; ++i) {
+    const int rr = row_of_rank<RPG>(my_rank, i, grp);  // this group's row inside the chunk
     const uint32_t first = __shfl_sync(0xffffffffu, rw.x, rr), cnt = __shfl_sync(0xffffffffu, rw.y, rr);
     const uint32_t cnt_max = __reduce_max_sync(0xffffffffu, cnt);
     float2 ao[CH * 4], ao2[CH * 4];
@@ -219,10 +225,14 @@ int fwd_t(const simt::Params& p, cudaStream_t st) {
   rp.B = p.B; rp.Hq = p.Hq; rp.Hkv = p.Hkv; rp.N = p.N; rp.Dg = p.D;
   rp.alpha = p.alpha;
   rp.sv = sup::view(p.support, nullptr, p.B, p.Hq, p.Hkv, p.N);
-  const long long warps = (long long)p.B * p.Hq * ((p.N + kRowsPerWarp - 1) / kRowsPerWarp);
+  // fewer than four CTAs per SM at 32 rows per warp: eight rows per warp
+  const bool small = (long long)p.B * p.Hq * p.N < 4LL * 148 * kRowsPerWarp * (kRowThreads / 32);
+  const int rows_w = small ? 8 : kRowsPerWarp;
+  const long long warps = (long long)p.B * p.Hq * ((p.N + rows_w - 1) / rows_w);
   const unsigned grid = (unsigned)((warps + kRowThreads / 32 - 1) / (kRowThreads / 32));
-  if (p.D > 64) fwd_rows_kernel<T, 2><<<grid, kRowThreads, 0, st>>>(rp);
-  else fwd_rows_kernel<T, 1><<<grid, kRowThreads, 0, st>>>(rp);
+  auto kernel = p.D > 64 ? (small ? fwd_rows_kernel<T, 2, 2> : fwd_rows_kernel<T, 2, 8>)
+                         : (small ? fwd_rows_kernel<T, 1, 2> : fwd_rows_kernel<T, 1, 8>);
+  kernel<<<grid, kRowThreads, 0, st>>>(rp);
   return check_launch("sparse::fwd_rows");
 }
 
@@ -426,26 +436,33 @@ __global__ void __launch_bounds__(kBwdRowThreads) bwd_rows_kernel(BwdParams p) {
 // Backward, by keys: dK, dV of 64 keys per CTA.
 // ---------------------------------------------------------------------------
 // Eight warps; warp w owns keys 4w .. 4w+3 of the CTA's 32, eight lanes per key, each lane D/8
-// elements of that key's dK and dV in registers.  For each query head of the group and each
-// 256-row block from the diagonal on, a thread reads where the block's entries of these 32 keys
-// lie in the block's sorted run (the row kernel left a table); the warps copy those segments to
-// shared memory at the offsets a
-// block-wide scan gives them -- the order (head, row block, key, row) is fixed -- and the staged
-// entries are regrouped by key with a stable counting sort.  The eight lanes of a key then run
-// through the key's range four entries at a time (the Q / dO rows of all four requested before
-// the first is used) and add P^T dO_i and dS^T Q_i.  No atomics: every sum has a fixed order.
+// elements of that key's dK and dV in registers.  The entries of these 32 keys lie in one segment
+// of each 256-row block's sorted run, for every query head of the group and each row block from
+// the diagonal on (the row kernel left a table).  A batch is up to kSegs segments, heads after
+// one another; a block-wide scan of their lengths gives every entry its place in the order
+// (head, row block, key, row), and a round fetches kStage of them to shared memory, each thread
+// looking up by bisection which segment its places belong to -- so that all loads of a round are in
+// flight together, however the entries are spread over segments.  (Copying segment by segment cost an L2
+// round trip per segment and warp: with 8 heads of 256 row blocks per key head, most of the kernel.)
+// The staged entries are regrouped by key with a stable counting sort.  The eight lanes of a
+// key then run through the key's range four entries at a time (the Q / dO rows of all four
+// requested before the first is used) and add P^T dO_i and dS^T Q_i.  No atomics: every sum has
+// a fixed order.
 constexpr int kKeyThreads = 256;
 constexpr int kKeyWarps = kKeyThreads / 32;
 constexpr int kKeysPerCta = sup::kTableKeys;  // 32: two CTAs fit an SM, and one's serial phases overlap the other's walk
 constexpr int kStage = 1024;  // entries staged per round
+constexpr int kSegPerThread = 4;
+constexpr int kSegs = kKeyThreads * kSegPerThread;  // segments per batch
+constexpr long long kMaxStagedRow = 1LL << 26;      // a staged entry's row (over the heads of a batch) has 26 bits
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
   constexpr int CH = D / 64;  // 16-byte loads per lane and row
-  __shared__ uint2 s_ent[kStage];       // ((absolute row << 6) | key inside the block, P^T | dS^T << 16)
+  __shared__ uint2 s_ent[kStage];       // ((row over the batch's heads << 6) | key inside the block, P^T | dS^T << 16)
   __shared__ uint2 s_srt[kStage];       // the same, regrouped by key
   __shared__ uint32_t s_wsum[kKeyWarps];
-  __shared__ uint32_t s_src[kKeyThreads], s_cnt[kKeyThreads], s_off[kKeyThreads];  // one segment per row block
+  __shared__ uint32_t s_src[kSegs], s_off[kSegs];  // a segment's first entry in by_key, its place in the batch
   __shared__ uint32_t s_kcnt[kKeysPerCta], s_kpos[kKeysPerCta + 1];
   __shared__ uint16_t s_ccnt[(kStage / 32) * kKeysPerCta];  // [chunk of 32 staged entries][key]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -469,23 +486,33 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
     const uint16_t hv = (uint16_t)bits16v;
     return __half2float(*reinterpret_cast<const __half*>(&hv));
   };
-  for (int g = 0; g < G; ++g) {
-    const int bh = b * p.Hq + kvh * G + g;
+  // causal: rows >= key, so the first row block that can hold these keys is the one of key0
+  const int c_first = p.causal ? (int)key0 / sup::kBlockRows : 0;
+  const int c_per_head = max(0, blocks_used - c_first);
+  const int g_step = (int)min((long long)G, max(1LL, kMaxStagedRow / p.N));  // heads whose rows a staged entry can name
+  for (int g0 = 0; g0 < G; g0 += g_step) {
+    const int gn = min(g_step, G - g0);
+    const int bh0 = b * p.Hq + kvh * G + g0;
     // the eight lanes of a key read 128 contiguous bytes of a row per load
-    const T* qh = (const T*)p.q + (size_t)bh * p.N * D + gl * 8;
-    const T* gh = (const T*)p.dout + (size_t)bh * p.N * D + gl * 8;
-    // causal: rows >= key, so the first row block that can hold these keys is the one of key0
-    for (int c0 = p.causal ? (int)key0 / sup::kBlockRows : 0; c0 < blocks_used; c0 += kKeyThreads) {
-      const int c = c0 + (int)threadIdx.x;
-      uint32_t lo = 0, hi = 0, src0 = 0;
-      if (c < blocks_used) {
-        const size_t bi = (size_t)bh * blocks + c;
-        const uint16_t* tab = p.sv.kb_off + bi * nkb1 + kb;
-        lo = tab[0]; hi = tab[1];
-        src0 = p.sv.blocks[bi].x + lo;
+    const T* qh = (const T*)p.q + (size_t)bh0 * p.N * D + gl * 8;
+    const T* gh = (const T*)p.dout + (size_t)bh0 * p.N * D + gl * 8;
+    const int n_segs = gn * c_per_head;
+    for (int c0 = 0; c0 < n_segs; c0 += kSegs) {
+      uint32_t src0[kSegPerThread], n_seg[kSegPerThread], n_mine = 0;
+#pragma unroll
+      for (int i = 0; i < kSegPerThread; ++i) {
+        const int c = c0 + (int)threadIdx.x * kSegPerThread + i;
+        src0[i] = 0; n_seg[i] = 0;
+        if (c < n_segs) {
+          const size_t bi = (size_t)(bh0 + c / c_per_head) * blocks + c_first + c % c_per_head;
+          const uint16_t* tab = p.sv.kb_off + bi * nkb1 + kb;
+          const uint32_t lo = tab[0], hi = tab[1];
+          n_seg[i] = hi - lo;
+          src0[i] = p.sv.blocks[bi].x + lo;
+        }
+        n_mine += n_seg[i];
       }
       // block-wide exclusive scan of the counts: where each thread's entries go
-      const uint32_t n_mine = hi - lo;
       uint32_t incl = n_mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -494,8 +521,6 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
       }
       __syncthreads();  // the previous batch has been walked
       if (lane == 31) s_wsum[warp] = incl;
-      s_src[threadIdx.x] = src0;
-      s_cnt[threadIdx.x] = n_mine;
       __syncthreads();
       uint32_t off = incl - n_mine, total = 0;
 #pragma unroll
@@ -504,22 +529,28 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
         off += (w < warp) ? t : 0u;
         total += t;
       }
-      s_off[threadIdx.x] = off;
-      const int n_here = min(kKeyThreads, blocks_used - c0);
+#pragma unroll
+      for (int i = 0; i < kSegPerThread; ++i) {
+        s_src[threadIdx.x * kSegPerThread + i] = src0[i];
+        s_off[threadIdx.x * kSegPerThread + i] = off;
+        off += n_seg[i];
+      }
       for (uint32_t r0 = 0; r0 < total; r0 += kStage) {
         __syncthreads();  // the segment table is written / the previous round has been walked
-        // a warp copies a segment, 32 entries per trip (segments of the first row blocks are long:
-        // their rows see few keys)
-        for (int t = warp; t < n_here; t += kKeyWarps) {
-          const uint32_t n = s_cnt[t], o = s_off[t];
-          const uint2* src = p.sv.by_key + s_src[t];
-          for (uint32_t e = lane; e < n; e += 32) {
-            const uint32_t pos = o + e - r0;  // wraps for entries of earlier rounds
-            if (pos < (uint32_t)kStage) {
-              const uint2 ent = src[e];
-              const uint32_t row = (uint32_t)(c0 + t) * sup::kBlockRows + (ent.x & 255u);
-              s_ent[pos] = make_uint2((row << 6) | ((ent.x >> 8) - key0), ent.y);
-            }
+#pragma unroll
+        for (int i = 0; i < kStage / kKeyThreads; ++i) {
+          const uint32_t pos = (uint32_t)(i * kKeyThreads) + threadIdx.x;
+          if (r0 + pos < total) {
+            // the last segment that starts at or before this place (the empty ones before it do not count:
+            // of equal starts the last is the one with the entry)
+            int lo = 0;
+#pragma unroll
+            for (int step = kSegs / 2; step > 0; step >>= 1)
+              if (s_off[lo + step] <= r0 + pos) lo += step;
+            const uint2 ent = p.sv.by_key[s_src[lo] + (r0 + pos - s_off[lo])];
+            const int c = c0 + lo;
+            const uint32_t row = (uint32_t)(c / c_per_head) * (uint32_t)p.N + (uint32_t)(c_first + c % c_per_head) * sup::kBlockRows + (ent.x & 255u);
+            s_ent[pos] = make_uint2((row << 6) | ((ent.x >> 8) - key0), ent.y);
           }
         }
         __syncthreads();

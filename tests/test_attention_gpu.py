@@ -434,6 +434,32 @@ def test_c_abi_error_codes_on_device():
     assert rc == 1 and b"unknown path" in lib.adasplash_last_error_string()
 
 
+@pytest.mark.parametrize("case", [
+    (2, 32, 4, 2048, 64, None), (2, 20, 4, 2048, 128, [2048, 900]),   # enough rows for 32 rows per warp of the forward
+    (1, 8, 1, 33000, 64, [33000]),   # more segments per key head than one batch of the key kernel; three sorting warps
+    (1, 2, 1, 65536, 128, None),     # the longest the supports cover: two sorting warps
+])
+def test_row_supports_on_large_problems(case):
+    B, Hq, Hkv, N, D, vl = case
+    q, k, v, do = (_randn(s, 90 + i, 1.5 if i < 2 else 1.0, torch.bfloat16).cuda() for i, s in
+                   enumerate([(B, Hq, N, D), (B, Hkv, N, D), (B, Hkv, N, D), (B, Hq, N, D)]))
+    varlen = None if vl is None else torch.tensor(vl, dtype=torch.int32).cuda()
+    _lib.set_kernel_path("tcgen05")
+    sup = att.support_buffer(att.make_shape(q, k, 1, varlen), q.device)
+    taus, bm = att.solve(q, k, 1, varlen, support=sup)
+    assert int((sup[256:256 + 4 * B * Hkv].view(torch.int32) == 0).sum()) == B * Hkv
+    out, out2 = att.forward_raw(q, k, v, taus, bm, varlen, support=sup)
+    ref, ref2 = att.forward_raw(q, k, v, taus, bm, varlen)
+    a = att.backward_raw(q, k, v, do, out2, taus, bm, varlen, 1, support=sup)
+    a2 = att.backward_raw(q, k, v, do, out2, taus, bm, varlen, 1, support=sup)
+    r = att.backward_raw(q, k, v, do, ref2, taus, bm, varlen, 1)
+    # 16-bit results of the same products in another order: as test_row_supports_match_tile_kernels
+    for name, x, y in (("out", out, ref), ("out2", out2, ref2), ("dq", a[0], r[0]), ("dk", a[1], r[1]), ("dv", a[2], r[2])):
+        assert (x.float() - y.float()).abs().max().item() < 1e-2 * max(1.0, y.float().abs().max().item()), name
+    for x, y in zip(a[:3], a2[:3]):
+        assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("D", [16, 32, 64, 128, 256])
 @pytest.mark.parametrize("scale", [0.05, 1.0, 3.0])
 @pytest.mark.parametrize("N,vl", [(256, [1, 193]), (512, None)])
