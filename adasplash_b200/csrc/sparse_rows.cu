@@ -267,11 +267,13 @@ __device__ __forceinline__ float group_sum8(float x) {  // over the eight lanes 
 //   p(u) = u^(1/(alpha-1)), g(u) = u^(1/(alpha-1) - 1): u^2 and u for alpha = 1.5.
 // Same warp layout as the forward gather: 32 rows per warp, eight lanes per row; the eight warps
 // of a CTA take the 256 rows of one solver CTA, whose entries form one contiguous run.  The
-// key-side values go to shared memory at the entry's slot, are sorted there by (key, row) once
+// key-side values go to shared memory at the entry's slot, are sorted by 32-key block once
 // the 256 rows are done, and leave as the block's run of `by_key`.
+constexpr int kSortCounters = 4096;  // 16-bit counters of the sort: 8 KB, so that three CTAs fit an SM
+
 template <typename T, int CH>
 __global__ void __launch_bounds__(kBwdRowThreads) bwd_rows_kernel(BwdParams p) {
-  extern __shared__ uint2 sort_buf[];  // [kBlockCap]
+  extern __shared__ uint2 sort_buf[];  // [kBlockCap], then the sort's counters
   __shared__ uint32_t s_tot[kBwdRowThreads / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane >> 3, gl = lane & 7;
@@ -393,43 +395,82 @@ __global__ void __launch_bounds__(kBwdRowThreads) bwd_rows_kernel(BwdParams p) {
       }
     }
   }
-  // sort the block's entries by (key, row): bitonic network over the next power of two
+  // Sort the block's entries by 32-key block, the rows of a block in order (what the key kernel
+  // needs: it regroups by key, stably, itself): a stable counting sort.  Warp w of the sorting
+  // warps takes the w-th stretch of the entries, counts its entries per key block, and -- after a
+  // scan over (key block, warp) -- hands out their places in the same order.  (A bitonic network over
+  // (key, row) kept shared memory busy for 30 % of this kernel's time.)
   __syncthreads();
   uint32_t total = 0;
 #pragma unroll
   for (int w = 0; w < kBwdRowThreads / 32; ++w) total += s_tot[w];
   total = min(total, (uint32_t)sup::kBlockCap);  // the solver exports no denser block
-  uint32_t n2 = 64;
-  while (n2 < total) n2 <<= 1;
-  for (uint32_t t = total + threadIdx.x; t < n2; t += kBwdRowThreads) sb[t] = make_uint2(0xffffffffu, 0u);
+  const int nkb = (p.N + sup::kTableKeys - 1) / sup::kTableKeys;
+  const int sort_warps = min(kBwdRowThreads / 32, kSortCounters / nkb);  // N <= 65536: at least two
+  uint16_t* cnt = reinterpret_cast<uint16_t*>(sort_buf + sup::kBlockCap);  // [sorting warp][key block]
+  for (int t = threadIdx.x; t < sort_warps * nkb; t += kBwdRowThreads) cnt[t] = 0;
   __syncthreads();
-  for (uint32_t k = 2; k <= n2; k <<= 1) {
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t pi = threadIdx.x; pi < n2 / 2; pi += kBwdRowThreads) {  // the pi-th pair (t, t | j) of this stage
-        const uint32_t t = ((pi & ~(j - 1)) << 1) | (pi & (j - 1)), x = t | j;
-        const uint2 a = sb[t], c = sb[x];
-        const bool up = (t & k) == 0;
-        if (up ? a.x > c.x : a.x < c.x) { sb[t] = c; sb[x] = a; }
+  const uint32_t stretch = (total + 32 * sort_warps - 1) / (32 * sort_warps) * 32;
+  uint16_t* my_cnt = cnt + warp * nkb;
+  auto walk = [&](auto&& f) {
+    if (warp >= sort_warps) return;
+    const uint32_t e1 = min(total, (warp + 1) * stretch);
+    for (uint32_t e = warp * stretch; e < e1; e += 32) {
+      const bool in = e + lane < e1;
+      const uint2 ent = in ? sb[e + lane] : make_uint2(0u, 0u);
+      const uint32_t bin = in ? ent.x >> 13 : 0x80000000u + lane;  // key / 32; idle lanes match nobody
+      const uint32_t same = __match_any_sync(0xffffffffu, bin);
+      f(ent, bin, in, (uint32_t)__popc(same & ((1u << lane) - 1u)), (uint32_t)__popc(same));
+      __syncwarp();
+    }
+  };
+  static_assert(sup::kTableKeys == 32, "the key block of an entry is its key's upper bits");
+  walk([&](const uint2&, uint32_t bin, bool in, uint32_t rank, uint32_t n) {
+    if (in && rank == 0u) my_cnt[bin] += (uint16_t)n;
+  });
+  __syncthreads();
+  {
+    // where each key block starts in the sorted run goes to the key kernel's table as well
+    const int per = (nkb + kBwdRowThreads - 1) / kBwdRowThreads;
+    const int k0 = min(nkb, (int)threadIdx.x * per), k1 = min(nkb, k0 + per);
+    uint32_t mine = 0;
+    for (int w = 0; w < sort_warps; ++w)
+      for (int k = k0; k < k1; ++k) mine += cnt[w * nkb + k];
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    __shared__ uint32_t s_scan[kBwdRowThreads / 32];
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - mine;
+#pragma unroll
+    for (int w = 0; w < kBwdRowThreads / 32; ++w) at += w < warp ? s_scan[w] : 0u;
+    uint16_t* tab = p.sv.kb_off + ((size_t)bh * blocks + blk) * (nkb + 1);
+    for (int k = k0; k < k1; ++k) {
+      tab[k] = (uint16_t)at;
+      for (int w = 0; w < sort_warps; ++w) {
+        const uint32_t c = cnt[w * nkb + k];
+        cnt[w * nkb + k] = (uint16_t)at;
+        at += c;
       }
-      // With distances up to 32 a warp's pairs lie in 64-element windows that no other warp
-      // touches, so stages at those distances only need the warp in step.
-      const uint32_t jn = j > 1 ? (j >> 1) : k;  // the distance of the stage that follows
-      if (j > 32 || jn > 32) __syncthreads(); else __syncwarp();
+    }
+    if (threadIdx.x == 0) {
+      tab[nkb] = (uint16_t)total;
+      p.sv.blocks[(size_t)bh * blocks + blk] = make_uint2(run0, total);
     }
   }
   __syncthreads();
-  for (uint32_t t = threadIdx.x; t < total; t += kBwdRowThreads) p.sv.by_key[run0 + t] = sb[t];
-  if (threadIdx.x == 0) p.sv.blocks[(size_t)bh * blocks + blk] = make_uint2(run0, total);
-  // where each 32-key block starts in the sorted run: the key kernel reads its bounds from this
-  // table instead of searching the run in global memory
-  const int nkb1 = (p.N + sup::kTableKeys - 1) / sup::kTableKeys + 1;
-  uint16_t* tab = p.sv.kb_off + ((size_t)bh * blocks + blk) * nkb1;
-  for (int kbi = threadIdx.x; kbi < nkb1; kbi += kBwdRowThreads) {
-    const uint32_t key = (uint32_t)(kbi * sup::kTableKeys) << 8;
-    uint32_t a = 0, z = total;
-    while (a < z) { const uint32_t m = (a + z) >> 1; if (sb[m].x < key) a = m + 1; else z = m; }
-    tab[kbi] = (uint16_t)a;
-  }
+  walk([&](const uint2& ent, uint32_t bin, bool in, uint32_t rank, uint32_t n) {
+    const uint32_t first = in ? my_cnt[bin] : 0u;
+    __syncwarp();
+    if (in) {
+      p.sv.by_key[run0 + first + rank] = ent;
+      if (rank == 0u) my_cnt[bin] = (uint16_t)(first + n);
+    }
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -681,7 +722,7 @@ int bwd_t(const simt::Params& p, cudaStream_t st) {
   bp.sv = sup::view(p.support, p.bwd_scratch, p.B, p.Hq, p.Hkv, p.N);
   static_assert(sup::kBlockRows == (kBwdRowThreads / 32) * kRowsPerWarp, "one CTA per row block");
   const unsigned grid = (unsigned)((long long)p.B * p.Hq * ((p.N + sup::kBlockRows - 1) / sup::kBlockRows));
-  const size_t sm = (size_t)sup::kBlockCap * sizeof(uint2);
+  const size_t sm = (size_t)sup::kBlockCap * sizeof(uint2) + kSortCounters * sizeof(uint16_t);
   auto rows_kernel = p.D > 64 ? bwd_rows_kernel<T, 2> : bwd_rows_kernel<T, 1>;
   {
     static std::mutex mu;

@@ -16,7 +16,7 @@
 //
 // The backward needs the same pairs by key as well (dK_j and dV_j sum over the rows that
 // attend to key j).  Its row kernel leaves, for every 256-row block (the rows of one solver CTA),
-// the block's entries sorted by (key, row) -- in the same slots of a second array -- and the key
+// the block's entries sorted by 32-key block, rows in order -- in the same slots of a second array -- and the key
 // kernel finds the entries of its keys in each block through a table the row kernel leaves beside the run: no atomics, and a
 // fixed summation order.
 //
@@ -33,7 +33,7 @@
 //   entries  uint2 [cap]: (key index, fp32 bits of u = z - tau_final > 0)
 // and of the backward's scratch (workspace + 256):
 //   by_key   uint2 [cap]: (key << 8 | row inside its 256-row block, P^T | dS^T << 16 as 16-bit
-//            values), each block's run sorted ascending; written by the backward
+//            values), each block's run sorted by 32-key block, rows in order; written by the backward
 //   blocks   uint2 [B*Hq*ceil(N/256)]: (first entry of the block's run, its length)
 //   kb_off   uint16 [B*Hq*ceil(N/256)][ceil(N/32)+1]: where the entries of each 32-key block
 //            (the keys of one CTA of the key kernel) start inside a row block's sorted run (the
