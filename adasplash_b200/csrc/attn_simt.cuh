@@ -649,51 +649,51 @@ __global__ void __launch_bounds__(kThreads) fwd_kernel(Params p) {
 // delta[row] = sum_d out2[row,d] * dO[row,d] in fp32 (adasplash_v2.py:838-898)
 // HBM-bound: every lane moves 16 bytes per load, D*sizeof(T)/16 lanes share a row (D is a
 // power of two >= 16, so that count is a power of two), and a warp keeps kDeltaUnroll groups
-// of rows in flight.
+// of rows in flight.  A CTA stays inside one head and walks its rows in steps, so that a head the
+// gather kernels own (support.cuh) costs kDeltaCtas CTAs that look at one flag.
 constexpr int kDeltaUnroll = 4;
 constexpr int kDeltaThreads = 256;
+constexpr int kDeltaCtas = 16;  // most CTAs per head, unless that leaves fewer than eight per SM
 
 template <typename T>
-__host__ __device__ constexpr int delta_rows_per_warp(int D) {
+__host__ __device__ constexpr int delta_rows_per_cta(int D) {
   const int vec = 16 / (int)sizeof(T);
   const int lpr = D / vec < 32 ? D / vec : 32;   // lanes per row
-  return (32 / lpr) * kDeltaUnroll;
+  return (32 / lpr) * kDeltaUnroll * (kDeltaThreads / 32);
+}
+template <typename T>
+inline int delta_ctas_per_head(int heads, int N, int D) {
+  const int n = (N + delta_rows_per_cta<T>(D) - 1) / delta_rows_per_cta<T>(D);
+  const int most = 8 * 148 / heads > kDeltaCtas ? 8 * 148 / heads : kDeltaCtas;
+  return n < most ? n : most;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kDeltaThreads)
 bwd_delta_kernel(const T* __restrict__ o2, const T* __restrict__ dout, float* __restrict__ delta,
-                 const void* varlen, int is_i64, int B, int H, int N, int D,
+                 const void* varlen, int is_i64, int H, int N, int D, int ctas_per_head,
                  const int32_t* __restrict__ skip = nullptr, int Hkv = 1) {
   constexpr int VEC = 16 / (int)sizeof(T);
+  const int hd = blockIdx.x / ctas_per_head, part = blockIdx.x % ctas_per_head;
+  const int b = hd / H;
+  if (skip != nullptr && skip[b * Hkv + (hd % H) / (H / Hkv)] == 0) return;
   const int chunks = D / VEC;                     // 16-byte chunks per row
   const int lpr = chunks < 32 ? chunks : 32;      // lanes per row
   const int rows_pass = 32 / lpr;                 // rows a warp covers per pass
   const int lane = threadIdx.x & 31;
   const int sub = lane / lpr, li = lane % lpr;
-  const long long total = (long long)B * H * N;
-  const long long warp_id = (long long)blockIdx.x * (kDeltaThreads / 32) + threadIdx.x / 32;
-  const long long row0 = warp_id * (rows_pass * kDeltaUnroll);
-  if (skip != nullptr && row0 < total) {
-    // the warp's rows lie in one head or two neighbours: leave if the gather kernels own both
-    const long long last = min(total, row0 + rows_pass * kDeltaUnroll) - 1;
-    const long long h0 = row0 / N, h1 = last / N;
-    const int G = H / Hkv;
-    if (h1 - h0 <= 1 && skip[(h0 / H) * Hkv + (h0 % H) / G] == 0 && skip[(h1 / H) * Hkv + (h1 % H) / G] == 0) return;
-  }
-  float acc[kDeltaUnroll];
+  const int len = load_len(varlen, is_i64, b, N);
+  const int step = rows_pass * kDeltaUnroll * (kDeltaThreads / 32);  // rows per CTA and turn
+  const long long base = (long long)hd * N;
+  for (int row0 = part * step + (threadIdx.x / 32) * (rows_pass * kDeltaUnroll); row0 < N; row0 += ctas_per_head * step) {
+    float acc[kDeltaUnroll];
 #pragma unroll
-  for (int u = 0; u < kDeltaUnroll; ++u) {
-    acc[u] = 0.f;
-    const long long row = row0 + u * rows_pass + sub;
-    if (row < total) {
-      const int b = (int)(row / ((long long)H * N));
-      const int r = (int)(row % N);
-      // heads of a kv head whose counter is zero belong to the gather kernels (support.cuh)
-      const bool mine = skip == nullptr || skip[b * Hkv + (int)((row / N) % H) / (H / Hkv)] != 0;
-      if (mine && r < load_len(varlen, is_i64, b, N)) {
-        const uint4* a = reinterpret_cast<const uint4*>(o2 + row * D);
-        const uint4* g = reinterpret_cast<const uint4*>(dout + row * D);
+    for (int u = 0; u < kDeltaUnroll; ++u) {
+      acc[u] = 0.f;
+      const int r = row0 + u * rows_pass + sub;
+      if (r < len) {
+        const uint4* a = reinterpret_cast<const uint4*>(o2 + (base + r) * D);
+        const uint4* g = reinterpret_cast<const uint4*>(dout + (base + r) * D);
         for (int c = li; c < chunks; c += lpr) {
           const uint4 va = a[c], vg = g[c];
           const T* ea = reinterpret_cast<const T*>(&va);
@@ -703,13 +703,13 @@ bwd_delta_kernel(const T* __restrict__ o2, const T* __restrict__ dout, float* __
         }
       }
     }
-  }
 #pragma unroll
-  for (int u = 0; u < kDeltaUnroll; ++u) {
-    float s = acc[u];
-    for (int o = lpr >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const long long row = row0 + u * rows_pass + sub;
-    if (li == 0 && row < total) delta[row] = s;
+    for (int u = 0; u < kDeltaUnroll; ++u) {
+      float s = acc[u];
+      for (int o = lpr >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const int r = row0 + u * rows_pass + sub;
+      if (li == 0 && r < N) delta[base + r] = s;
+    }
   }
 }
 

@@ -100,11 +100,9 @@ int bwd_t(const simt::Params& p, void* ws, cudaStream_t st) {
   // with a row-support buffer, heads the gather kernels own are skipped by every kernel here
   const int32_t* skip = p.support != nullptr ? sup::view(p.support, nullptr, p.B, p.Hq, p.Hkv, p.N).dense : nullptr;
   if (stages & ADS_BWD_DELTA) {
-    long long rows = (long long)p.B * p.Hq * p.N;
-    const long long per_block = (long long)(simt::kDeltaThreads / 32) * simt::delta_rows_per_warp<T>(p.D);
-    unsigned grid = (unsigned)((rows + per_block - 1) / per_block);
-    simt::bwd_delta_kernel<T><<<grid, simt::kDeltaThreads, 0, st>>>((const T*)p.out2_in, (const T*)p.dout, p.delta,
-                                                    p.varlen, p.varlen_is_i64, p.B, p.Hq, p.N, p.D, skip, p.Hkv);
+    const int per_head = simt::delta_ctas_per_head<T>(p.B * p.Hq, p.N, p.D);
+    simt::bwd_delta_kernel<T><<<(unsigned)((long long)p.B * p.Hq * per_head), simt::kDeltaThreads, 0, st>>>(
+        (const T*)p.out2_in, (const T*)p.dout, p.delta, p.varlen, p.varlen_is_i64, p.Hq, p.N, p.D, per_head, skip, p.Hkv);
     if (int rc = check_launch("sm100::bwd_delta")) return rc;
   }
   if (stages & ADS_BWD_TRANSPOSE) {
