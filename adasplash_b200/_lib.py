@@ -6,11 +6,14 @@ an exception is raised.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import threading
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int32, c_int64, c_size_t, c_void_p
 from pathlib import Path
+
+import torch
 
 LIB_PATH = Path(__file__).resolve().parent / "_C" / "libadasplash_b200.so"
 
@@ -100,12 +103,27 @@ def kernel_path() -> int:
     return _PATH_NAMES[name]
 
 
+_DTYPE_CODES = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
+
+
 def dtype_code(dtype) -> int:
-    import torch
     try:
-        return {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}[dtype]
+        return _DTYPE_CODES[dtype]
     except KeyError:
         raise AssertionError(f"unsupported dtype {dtype}; expected float32, float16 or bfloat16")
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def on_device(device):
+    """Context in which `device` is the current one; nothing to enter where it already is."""
+    return _NO_GUARD if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def stream_ptr(device) -> int:
+    """The handle of torch's current stream on `device`."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def launch_count() -> int:

@@ -9,6 +9,7 @@ nothing here synchronises the host.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -49,13 +50,15 @@ def _check_inputs(q, k, v, varlen, require_pow2=True, min_len=BMASK_TILE):
         "q, k and v must be CUDA tensors on one device (there is no CPU path)")
 
 
-def make_shape(q, k, niter, varlen, path=None, alpha=1.5, is_causal=True):
+def _shape_key(q, k, niter, varlen, path, alpha, is_causal):
     B, Hq, N, D = q.shape
-    return _lib.AttnShape(
-        B=B, Hq=Hq, Hkv=k.shape[1], N=N, D=D, dtype=_lib.dtype_code(q.dtype), niter=int(niter),
-        varlen_is_i64=int(varlen is not None and varlen.dtype == torch.int64),
-        path=_lib.kernel_path() if path is None else path,
-        alpha=float(alpha), non_causal=int(not is_causal))
+    return (B, Hq, k.shape[1], N, D, _lib.dtype_code(q.dtype), int(niter),
+            int(varlen is not None and varlen.dtype == torch.int64),
+            _lib.kernel_path() if path is None else path, 0, float(alpha), int(not is_causal))
+
+
+def make_shape(q, k, niter, varlen, path=None, alpha=1.5, is_causal=True):
+    return _lib.AttnShape(*_shape_key(q, k, niter, varlen, path, alpha, is_causal))
 
 
 def bitmap_extent(shape):
@@ -64,15 +67,39 @@ def bitmap_extent(shape):
     return rows.value, words.value
 
 
-def _workspace(shape, device, full=False):
-    """Scratch of one call: the 256-byte status word; `full` (a backward with a support buffer)
-    adds the room for its key-sorted copy of the supports."""
-    nbytes = int(_lib.load().adasplash2_workspace_bytes(ctypes.byref(shape)))
-    if nbytes == 0:
-        _lib.check(_lib.load().adasplash2_resolved_path(ctypes.byref(shape)) < 0)
-    if not full:
-        nbytes = min(nbytes, 256)
-    return torch.empty(max(nbytes, 256), device=device, dtype=torch.uint8), nbytes
+class _Plan:
+    """What a call needs to know of its shape, asked of the library once per shape: the sizes of
+    its buffers and the shape's C struct (shared by calls and threads: read only)."""
+    __slots__ = ("shape", "ref", "rows", "words", "ws_bytes", "sup_bytes")
+
+    def __init__(self, key):
+        lib = _lib.load()
+        self.shape = _lib.AttnShape(*key)
+        self.ref = ctypes.byref(self.shape)
+        self.rows, self.words = bitmap_extent(self.shape)
+        self.ws_bytes = int(lib.adasplash2_workspace_bytes(self.ref))
+        if self.ws_bytes == 0:
+            _lib.check(lib.adasplash2_resolved_path(self.ref) < 0)
+        self.sup_bytes = int(lib.adasplash2_support_bytes(self.ref))
+
+    def workspace(self, device, full=False):
+        """Scratch of one call: the 256-byte status word; `full` (a backward with a support buffer)
+        adds the room for its key-sorted copy of the supports."""
+        nbytes = self.ws_bytes if full else min(self.ws_bytes, 256)
+        return torch.empty(max(nbytes, 256), device=device, dtype=torch.uint8), nbytes
+
+    def support(self, device):
+        """Buffer for the rows' supports of one problem (None where the library has no such route)."""
+        if self.sup_bytes == 0 or not ROW_SUPPORTS:
+            return None
+        return torch.empty(self.sup_bytes, device=device, dtype=torch.uint8)
+
+
+_plan_of = functools.lru_cache(maxsize=256)(_Plan)
+
+
+def _plan(q, k, niter, varlen, path=None, alpha=1.5, is_causal=True):
+    return _plan_of(_shape_key(q, k, niter, varlen, path, alpha, is_causal))
 
 
 ROW_SUPPORTS = True   # let the solver export the rows' supports, so that sparse heads run as gathers
@@ -104,16 +131,15 @@ def solve(q, k, niter=1, varlen=None, path=None, alpha=1.5, is_causal=True, supp
     """Thresholds and block mask only: (taus (B,Hq,N) fp32, bmask int32).  `support`: a buffer
     from `support_buffer` that receives the rows' supports."""
     lib = _lib.load()
-    shape = make_shape(q, k, niter, varlen, path, alpha, is_causal)
-    rows, words = bitmap_extent(shape)
+    plan = _plan(q, k, niter, varlen, path, alpha, is_causal)
     B, Hq, N, _ = q.shape
     taus = torch.empty((B, Hq, N), device=q.device, dtype=torch.float32)
-    bmask = torch.empty((B, Hq, rows, words), device=q.device, dtype=torch.int32)
-    with torch.cuda.device(q.device):
-        ws, nbytes = _workspace(shape, q.device)
-        st = torch.cuda.current_stream().cuda_stream
+    bmask = torch.empty((B, Hq, plan.rows, plan.words), device=q.device, dtype=torch.int32)
+    with _lib.on_device(q.device):
+        ws, nbytes = plan.workspace(q.device)
+        st = _lib.stream_ptr(q.device)
         _lib.check(lib.adasplash2_solve(_ptr(q), _ptr(k), _ptr(varlen), _ptr(taus), _ptr(bmask),
-                                        ctypes.byref(shape), _ptr(ws), nbytes, *_sup_args(support), st))
+                                        plan.ref, _ptr(ws), nbytes, *_sup_args(support), st))
         _maybe_check(ws, st)
     return taus, bmask
 
@@ -121,16 +147,15 @@ def solve(q, k, niter=1, varlen=None, path=None, alpha=1.5, is_causal=True, supp
 def mask_from_tau(q, k, taus, varlen=None, path=None):
     """Block mask for caller-supplied thresholds (bit = any(z > tau) per 64x64 tile)."""
     lib = _lib.load()
-    shape = make_shape(q, k, 0, varlen, path)
-    rows, words = bitmap_extent(shape)
+    plan = _plan(q, k, 0, varlen, path)
     B, Hq, N, _ = q.shape
     assert taus.shape == (B, Hq, N) and taus.dtype == torch.float32 and taus.is_contiguous()
-    bmask = torch.empty((B, Hq, rows, words), device=q.device, dtype=torch.int32)
-    with torch.cuda.device(q.device):
-        ws, nbytes = _workspace(shape, q.device)
-        st = torch.cuda.current_stream().cuda_stream
+    bmask = torch.empty((B, Hq, plan.rows, plan.words), device=q.device, dtype=torch.int32)
+    with _lib.on_device(q.device):
+        ws, nbytes = plan.workspace(q.device)
+        st = _lib.stream_ptr(q.device)
         _lib.check(lib.adasplash2_mask_from_tau(_ptr(q), _ptr(k), _ptr(varlen), _ptr(taus),
-                                                _ptr(bmask), ctypes.byref(shape), _ptr(ws),
+                                                _ptr(bmask), plan.ref, _ptr(ws),
                                                 nbytes, st))
         _maybe_check(ws, st)
     return bmask
@@ -141,19 +166,18 @@ class _SparseAttention(torch.autograd.Function):
     def forward(ctx, q, k, v, niter=10, varlen=None):
         _check_inputs(q, k, v, varlen)
         lib = _lib.load()
-        shape = make_shape(q, k, niter, varlen)
-        rows, words = bitmap_extent(shape)
+        plan = _plan(q, k, niter, varlen)
         B, Hq, N, _ = q.shape
         dev = q.device
         taus = torch.empty((B, Hq, N), device=dev, dtype=torch.float32)
-        bmask = torch.empty((B, Hq, rows, words), device=dev, dtype=torch.int32)
+        bmask = torch.empty((B, Hq, plan.rows, plan.words), device=dev, dtype=torch.int32)
         out = torch.empty_like(q)
         out2 = torch.empty_like(q)
-        with torch.cuda.device(dev):
-            ws, nbytes = _workspace(shape, dev)
-            support = support_buffer(shape, dev) if N >= ROW_SUPPORTS_MIN_N else None
-            st = torch.cuda.current_stream().cuda_stream
-            sp = ctypes.byref(shape)
+        with _lib.on_device(dev):
+            ws, nbytes = plan.workspace(dev)
+            support = plan.support(dev) if N >= ROW_SUPPORTS_MIN_N else None
+            st = _lib.stream_ptr(dev)
+            sp = plan.ref
             _lib.check(lib.adasplash2_solve(_ptr(q), _ptr(k), _ptr(varlen), _ptr(taus),
                                             _ptr(bmask), sp, _ptr(ws), nbytes, *_sup_args(support), st))
             _maybe_check(ws, st)
@@ -182,14 +206,14 @@ def forward_raw(q, k, v, taus, bmask, varlen=None, path=None, alpha=1.5, is_caus
     """`adasplash2_fwd` alone for given thresholds and block mask: (out, out2).  `support`: the
     buffer a `solve` of the same problem filled."""
     lib = _lib.load()
-    shape = make_shape(q, k, 0, varlen, path, alpha, is_causal)
+    plan = _plan(q, k, 0, varlen, path, alpha, is_causal)
     out = torch.empty_like(q)
     out2 = torch.empty_like(q)
-    with torch.cuda.device(q.device):
-        ws, nbytes = _workspace(shape, q.device)
-        st = torch.cuda.current_stream().cuda_stream
+    with _lib.on_device(q.device):
+        ws, nbytes = plan.workspace(q.device)
+        st = _lib.stream_ptr(q.device)
         _lib.check(lib.adasplash2_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(varlen), _ptr(taus),
-                                      _ptr(bmask), _ptr(out), _ptr(out2), ctypes.byref(shape),
+                                      _ptr(bmask), _ptr(out), _ptr(out2), plan.ref,
                                       _ptr(ws), nbytes, *_sup_args(support), st))
         _maybe_check(ws, st)
     return out, out2
@@ -201,20 +225,24 @@ def backward_raw(q, k, v, do, out2, taus, bmask, varlen=None, niter=1, stages=0,
     the named kernels (ADS_BWD_* mask; a measurement aid), reusing `buffers` =
     (dq, dk, dv, delta, bmask_t) from an earlier full call."""
     lib = _lib.load()
-    shape = make_shape(q, k, niter, varlen, path, alpha, is_causal)
-    shape.bwd_stages = int(stages)
+    plan = _plan(q, k, niter, varlen, path, alpha, is_causal)
+    sp = plan.ref
+    if stages:
+        shape = make_shape(q, k, niter, varlen, path, alpha, is_causal)
+        shape.bwd_stages = int(stages)
+        sp = ctypes.byref(shape)
     dev = q.device
     if buffers is None:
         buffers = (torch.empty_like(q), torch.empty_like(k), torch.empty_like(v),
                    torch.empty(taus.shape, device=dev, dtype=torch.float32), torch.empty_like(bmask))
     dq, dk, dv, delta, bmask_t = buffers
-    with torch.cuda.device(dev):
-        ws, nbytes = _workspace(shape, dev, full=support is not None)
-        st = torch.cuda.current_stream().cuda_stream
+    with _lib.on_device(dev):
+        ws, nbytes = plan.workspace(dev, full=support is not None)
+        st = _lib.stream_ptr(dev)
         _lib.check(lib.adasplash2_bwd(_ptr(q), _ptr(k), _ptr(v), _ptr(do), _ptr(out2),
                                       _ptr(varlen), _ptr(taus), _ptr(bmask), _ptr(bmask_t),
                                       _ptr(delta), _ptr(dq), _ptr(dk), _ptr(dv),
-                                      ctypes.byref(shape), _ptr(ws), nbytes, *_sup_args(support), st))
+                                      sp, _ptr(ws), nbytes, *_sup_args(support), st))
         _maybe_check(ws, st)
     return dq, dk, dv, delta, bmask_t
 

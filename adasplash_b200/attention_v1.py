@@ -26,8 +26,7 @@ class _SparseAttentionV1(torch.autograd.Function):
         support = None
         if q.shape[2] >= att.ROW_SUPPORTS_MIN_N:
             # rows' supports from the solver: sparse heads run as gathers (see attention.py)
-            with torch.cuda.device(q.device):
-                support = att.support_buffer(att.make_shape(q, k, niter, varlen, None, alpha, is_causal), q.device)
+            support = att._plan(q, k, niter, varlen, None, alpha, is_causal).support(q.device)
         taus, bmask = att.solve(q, k, niter, varlen, None, alpha, is_causal, support=support)
         out, out2 = att.forward_raw(q, k, v, taus, bmask, varlen, None, alpha, is_causal, support=support)
         ctx.save_for_backward(q, k, v, out2, taus, bmask)

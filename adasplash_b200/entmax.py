@@ -24,8 +24,8 @@ class _EntmaxFunction(torch.autograd.Function):
         cols = x.shape[-1] if x.dim() > 0 else 1
         rows = x.numel() // cols if cols > 0 else 0
         y = torch.empty_like(x)
-        with torch.cuda.device(x.device):
-            st = torch.cuda.current_stream().cuda_stream
+        with _lib.on_device(x.device):
+            st = _lib.stream_ptr(x.device)
             _lib.check(lib.adasplash_entmax_fwd(
                 _ptr(x), _ptr(y), None, rows, cols, float(alpha), int(n_iter),
                 int(bool(use_histogram)), int(bool(fast_math)), _lib.dtype_code(x.dtype), st))
@@ -45,8 +45,8 @@ class _EntmaxFunction(torch.autograd.Function):
         cols = y.shape[-1] if y.dim() > 0 else 1
         rows = y.numel() // cols if cols > 0 else 0
         dx = torch.empty_like(y)
-        with torch.cuda.device(y.device):
-            st = torch.cuda.current_stream().cuda_stream
+        with _lib.on_device(y.device):
+            st = _lib.stream_ptr(y.device)
             _lib.check(lib.adasplash_entmax_bwd(
                 _ptr(y), _ptr(dy), _ptr(dx), rows, cols, ctx.alpha, int(ctx.fast_math),
                 _lib.dtype_code(y.dtype), st))
@@ -81,8 +81,8 @@ def entmax_with_tau(x, alpha=1.5, n_iter=2, use_histogram=True, fast_math=False)
     rows = x.numel() // cols
     y = torch.empty_like(x)
     tau = torch.empty(x.shape[:-1], device=x.device, dtype=torch.float32)
-    with torch.cuda.device(x.device):
-        st = torch.cuda.current_stream().cuda_stream
+    with _lib.on_device(x.device):
+        st = _lib.stream_ptr(x.device)
         _lib.check(lib.adasplash_entmax_fwd(
             _ptr(x), _ptr(y), _ptr(tau), rows, cols, float(alpha), int(n_iter),
             int(bool(use_histogram)), int(bool(fast_math)), _lib.dtype_code(x.dtype), st))
