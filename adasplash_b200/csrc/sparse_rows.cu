@@ -504,8 +504,10 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
   __shared__ uint2 s_srt[kStage];       // the same, regrouped by key
   __shared__ uint32_t s_wsum[kKeyWarps];
   __shared__ uint32_t s_src[kSegs], s_off[kSegs];  // a segment's first entry in by_key, its place in the batch
-  __shared__ uint32_t s_kcnt[kKeysPerCta], s_kpos[kKeysPerCta + 1];
-  __shared__ uint16_t s_ccnt[(kStage / 32) * kKeysPerCta];  // [chunk of 32 staged entries][key]
+  __shared__ uint32_t s_row[kSegs];                // and the row (over the heads of the batch) its block starts at
+  __shared__ uint32_t s_kcnt[kKeysPerCta];
+  constexpr int kPitch = kKeysPerCta + 2;  // rows of eight threads' chunks start four banks apart
+  __shared__ uint16_t s_ccnt[(kStage / 32) * kPitch];  // [chunk of 32 staged entries][key]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane >> 3, gl = lane & 7;
   const int nkb = (p.N + kKeysPerCta - 1) / kKeysPerCta;
@@ -539,13 +541,19 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
     const T* gh = (const T*)p.dout + (size_t)bh0 * p.N * D + gl * 8;
     const int n_segs = gn * c_per_head;
     for (int c0 = 0; c0 < n_segs; c0 += kSegs) {
-      uint32_t src0[kSegPerThread], n_seg[kSegPerThread], n_mine = 0;
+      const int n_here = min(kSegs, n_segs - c0);
+      const int spt = (n_here + kKeyThreads - 1) / kKeyThreads;   // consecutive segments per thread
+      int top = 1;                                                // half the bisection's range
+      while (2 * top < n_here) top *= 2;
+      uint32_t src0[kSegPerThread], n_seg[kSegPerThread], row0[kSegPerThread], n_mine = 0;
 #pragma unroll
       for (int i = 0; i < kSegPerThread; ++i) {
-        const int c = c0 + (int)threadIdx.x * kSegPerThread + i;
-        src0[i] = 0; n_seg[i] = 0;
-        if (c < n_segs) {
-          const size_t bi = (size_t)(bh0 + c / c_per_head) * blocks + c_first + c % c_per_head;
+        const int t = (int)threadIdx.x * spt + i, c = c0 + t;
+        src0[i] = 0; n_seg[i] = 0; row0[i] = 0;
+        if (i < spt && t < n_here) {
+          const int hd = c / c_per_head, cb = c_first + c - hd * c_per_head;  // head of the batch, row block
+          const size_t bi = (size_t)(bh0 + hd) * blocks + cb;
+          row0[i] = (uint32_t)hd * (uint32_t)p.N + (uint32_t)cb * sup::kBlockRows;
           const uint16_t* tab = p.sv.kb_off + bi * nkb1 + kb;
           const uint32_t lo = tab[0], hi = tab[1];
           n_seg[i] = hi - lo;
@@ -572,8 +580,12 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
       }
 #pragma unroll
       for (int i = 0; i < kSegPerThread; ++i) {
-        s_src[threadIdx.x * kSegPerThread + i] = src0[i];
-        s_off[threadIdx.x * kSegPerThread + i] = off;
+        const int t = (int)threadIdx.x * spt + i;
+        if (i < spt && t < n_here) {
+          s_src[t] = src0[i];
+          s_off[t] = off;
+          s_row[t] = row0[i];
+        }
         off += n_seg[i];
       }
       for (uint32_t r0 = 0; r0 < total; r0 += kStage) {
@@ -585,21 +597,20 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
             // the last segment that starts at or before this place (the empty ones before it do not count:
             // of equal starts the last is the one with the entry)
             int lo = 0;
-#pragma unroll
-            for (int step = kSegs / 2; step > 0; step >>= 1)
-              if (s_off[lo + step] <= r0 + pos) lo += step;
+            for (int step = top; step > 0; step >>= 1)
+              if (lo + step < n_here && s_off[lo + step] <= r0 + pos) lo += step;
             const uint2 ent = p.sv.by_key[s_src[lo] + (r0 + pos - s_off[lo])];
-            const int c = c0 + lo;
-            const uint32_t row = (uint32_t)(c / c_per_head) * (uint32_t)p.N + (uint32_t)(c_first + c % c_per_head) * sup::kBlockRows + (ent.x & 255u);
+            const uint32_t row = s_row[lo] + (ent.x & 255u);
             s_ent[pos] = make_uint2((row << 6) | ((ent.x >> 8) - key0), ent.y);
           }
         }
         __syncthreads();
         const uint32_t m = min((uint32_t)kStage, total - r0);
         // Regroup the staged entries by key, keeping their order inside a key (a stable counting
-        // sort over the 64 keys; entries with zero weights drop out): each key's entries then
+        // sort over the 32 keys; entries with zero weights drop out): each key's entries then
         // lie in one range of s_srt.  Per 32-entry chunk the lanes with the same key rank
-        // themselves with a match; a thread per key turns the chunks' counts into offsets.
+        // themselves with a match; eight threads per key turn the chunks' counts into offsets, and
+        // every warp scans the keys' totals for itself.  (A thread per key walked 32 chunks alone.)
         const uint32_t n_chunks = (m + 31) >> 5;
         uint2 held[kStage / 32 / kKeyWarps];
         uint32_t ranks[kStage / 32 / kKeyWarps];
@@ -615,46 +626,53 @@ __global__ void __launch_bounds__(kKeyThreads, 2) bwd_keys_kernel(BwdParams p) {
             const uint32_t ek = live ? (held[i].x & 63u) : (64u + (uint32_t)lane);  // dead lanes match nobody (keys are < 32)
             const uint32_t same = __match_any_sync(0xffffffffu, ek);
             ranks[i] = __popc(same & ((1u << lane) - 1u));
-            s_ccnt[c * kKeysPerCta + lane] = 0;
+            s_ccnt[c * kPitch + lane] = 0;
             __syncwarp();
-            if (live && ranks[i] == 0u) s_ccnt[c * kKeysPerCta + ek] = (uint16_t)__popc(same);
+            if (live && ranks[i] == 0u) s_ccnt[c * kPitch + ek] = (uint16_t)__popc(same);
           }
         }
         __syncthreads();
-        if (threadIdx.x < kKeysPerCta) {
-          uint32_t running = 0;
-          for (uint32_t c = 0; c < n_chunks; ++c) {
-            const uint32_t t = s_ccnt[c * kKeysPerCta + threadIdx.x];
-            s_ccnt[c * kKeysPerCta + threadIdx.x] = (uint16_t)running;
-            running += t;
-          }
-          s_kcnt[threadIdx.x] = running;
-        }
-        __syncthreads();
-        if (warp == 0) {
-          static_assert(kKeysPerCta == 32, "one key counter per lane");
-          const uint32_t cmine = s_kcnt[lane];
-          uint32_t incl2 = cmine;
+        {
+          static_assert(kKeyThreads == 8 * kKeysPerCta && kStage / 32 % 8 == 0, "eight threads per key");
+          constexpr int CPT = kStage / 32 / 8;  // chunks per thread
+          const uint32_t key = threadIdx.x >> 3, c0t = (threadIdx.x & 7) * CPT;
+          uint32_t before[CPT], sum = 0;
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xffffffffu, incl2, o);
-            if (lane >= o) incl2 += up;
+          for (int i = 0; i < CPT; ++i) {
+            before[i] = sum;
+            sum += c0t + i < n_chunks ? s_ccnt[(c0t + i) * kPitch + key] : 0u;
           }
-          s_kpos[lane] = incl2 - cmine;
-          if (lane == 31) s_kpos[kKeysPerCta] = incl2;
+          uint32_t incl8 = sum;
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl8, o, 8);
+            if (gl >= o) incl8 += up;
+          }
+#pragma unroll
+          for (int i = 0; i < CPT; ++i)
+            if (c0t + i < n_chunks) s_ccnt[(c0t + i) * kPitch + key] = (uint16_t)(incl8 - sum + before[i]);
+          if (gl == 7) s_kcnt[key] = incl8;
         }
         __syncthreads();
+        static_assert(kKeysPerCta == 32, "one key counter per lane");
+        const uint32_t kcnt = s_kcnt[lane];
+        uint32_t kpos = kcnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t up = __shfl_up_sync(0xffffffffu, kpos, o);
+          if (lane >= o) kpos += up;
+        }
+        kpos -= kcnt;
 #pragma unroll
         for (int i = 0; i < kStage / 32 / kKeyWarps; ++i) {
           const uint32_t c = (uint32_t)(warp + i * kKeyWarps);
-          if (c < n_chunks && held[i].y != 0u) {
-            const uint32_t ek = held[i].x & 63u;
-            s_srt[s_kpos[ek] + s_ccnt[c * kKeysPerCta + ek] + ranks[i]] = held[i];
-          }
+          const uint32_t ek = held[i].x & 31u;
+          const uint32_t first = __shfl_sync(0xffffffffu, kpos, ek);
+          if (c < n_chunks && held[i].y != 0u) s_srt[first + s_ccnt[c * kPitch + ek] + ranks[i]] = held[i];
         }
         __syncthreads();
-        uint32_t e = s_kpos[my_local];
-        const uint32_t e_end = s_kpos[my_local + 1];
+        uint32_t e = __shfl_sync(0xffffffffu, kpos, my_local);
+        const uint32_t e_end = e + __shfl_sync(0xffffffffu, kcnt, my_local);
         while (__any_sync(0xffffffffu, e < e_end)) {
           uint4 rq[4][CH], rg[4][CH];
           uint32_t ys[4];
