@@ -371,7 +371,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
     float mx = -1.0e3f, tau0 = 0.f;
     float cls[kSolveClasses];  // maxima of this thread's keys by position (see below)
 #pragma unroll
-    for (int c = 0; c < kSolveClasses; ++c) cls[c] = -1.0e3f;
+    for (int c = 0; c < kSolveClasses; ++c) cls[c] = -INFINITY;   // a class without a key counts nowhere
     float thr_list = 0.f;      // scores from here on go to the lists
     int cnt[8];
     HalleyState hs;
