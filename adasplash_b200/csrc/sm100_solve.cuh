@@ -84,24 +84,32 @@ enum SweepMode : int { kModeMax = 0, kModeHist = 1, kModeHalley = 2, kModeFinal 
 struct __align__(8) Cand { float z; uint16_t key; uint16_t next; };
 constexpr uint16_t kCandNil = 0xffff;
 
-// Shared memory: K stages, barriers, exchange buffers, bitmap staging, then the two Q tiles and
+// Shared memory: barriers, exchange buffers, bitmap staging, K stages, then the two Q tiles and
 // whatever is left of the budget.  The Q tiles are dead once Q~ sits in TMEM (before the first
 // append), so the candidate pool is their space plus that remainder (D = 128: ~110 KB, 14000
 // entries, 27 per thread on average).  Each row warp appends to its own sixteenth and hands
 // out its slots by a warp vote.
+// CTAs with more than kSolveLongTiles key tiles also take the last K stage for their pool, once
+// sweep 1 is through, and stream their later sweeps through two stages (35 entries per thread):
+// rows of 16384 unit-variance keys list 29 per thread, and most of their CTAs took the third sweep --
+// 32 heads on 8, 8 sequences of 4096 to 16384 keys: 21.3 -> 16.2 ms.  Rows of up to 8192 such keys
+// list 24 or so, and there two stages cost 2 to 3 % (128 heads of 8192, spread 1.5: 2.60 -> 2.68 ms).
 constexpr int kSolveSmemBudget = 225 * 1024;
+constexpr int kSolveLongTiles = 56;
 
 template <int D>
 struct SolveSmem {
   static constexpr int tile_bytes = (D / 64) * kPanelBytes;
-  static constexpr int k_off = 0;
-  static constexpr int bar_off = k_off + kSolveStages * tile_bytes;
+  static constexpr int bar_off = 0;
   static constexpr int n_bars = 2 + 2 * kSolveStages + 4 * kSolveBufs + 1;
   static constexpr int misc_off = bar_off + n_bars * 8;            // tmem base, abort flag, status, pool counters
   static constexpr int xchg_off = misc_off + 128;                  // [2 groups][2 halves][8][128] floats
   static constexpr int bits_off = xchg_off + 2 * 2 * 8 * 128 * 4;  // [4][n_words] words
-  static __host__ __device__ int q_off(int n_words) { return (bits_off + 4 * n_words * 4 + 1023) & ~1023; }  // two Q tiles
-  static __host__ __device__ int pool_entries(int n_words) { return (kSolveSmemBudget - 1024 - q_off(n_words)) / 8; }
+  static __host__ __device__ int k_off(int n_words) { return (bits_off + 4 * n_words * 4 + 1023) & ~1023; }
+  static __host__ __device__ int q_off(int n_words) { return k_off(n_words) + kSolveStages * tile_bytes; }  // two Q tiles
+  // `late`: K stages of the sweeps after the first; the pool follows them
+  static __host__ __device__ int pool_off(int n_words, int late) { return k_off(n_words) + late * tile_bytes; }
+  static __host__ __device__ int pool_entries(int n_words, int late) { return (kSolveSmemBudget - 1024 - pool_off(n_words, late)) / 8; }
   static size_t bytes(int) { return kSolveSmemBudget; }
 };
 
@@ -122,7 +130,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem + L::q_off(p.n_words);
-  uint8_t* sK = smem + L::k_off;
+  uint8_t* sK = smem + L::k_off(p.n_words);
   uint64_t* bars = (uint64_t*)(smem + L::bar_off);
   uint64_t* q_full = bars + 0;
   uint64_t* q_ready = bars + 1;
@@ -140,8 +148,6 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
   int* pool_common = (int*)(smem + L::misc_off + 24);  // third sweep: entries used (one counter for the CTA)
   float* xchg = (float*)(smem + L::xchg_off);
   uint32_t* s_bits = (uint32_t*)(smem + L::bits_off);
-  Cand* pool = (Cand*)sQ;  // the Q tiles are dead once Q~ is in TMEM (before the first append)
-  const int warp_pool = L::pool_entries(p.n_words) / 16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int heads = p.B * p.Hq;
@@ -160,6 +166,9 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
   const int T_a = full_attn ? T_all : qtA + 1;      // key tiles of A: 0 .. qtA
   const int T_k = full_attn ? T_all : (b_on ? qtB + 1 : T_a);  // key tiles streamed per sweep
   const int nsweeps = p.tau_given ? 1 : p.niter + 3;
+  const int late_stages = T_k > kSolveLongTiles ? kSolveStages - 1 : kSolveStages;
+  Cand* pool = (Cand*)(smem + L::pool_off(p.n_words, late_stages));
+  const int warp_pool = L::pool_entries(p.n_words, late_stages) / 16;
   // tiles streamed before the row warps decide (max sweep, histogram + collect sweep), and in
   // all if the candidate pool overflows (then the Halley .. final steps sweep S as well)
   const int total_first = p.tau_given ? T_k : 2 * T_k;
@@ -220,9 +229,9 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           ptx::tma_load_3d(sQ + t * L::tile_bytes + pn * kPanelBytes, &tmQ, q_full, pn * 64, m0 + t * kBlockM, bh);
       const int kv_head = b * p.Hkv + kvh;
       int total = total_first;
-      // stage, its use parity and the key tile are carried along (no divisions in the loop)
-      int st = 0, kt = 0;
-      uint32_t use_par = 0;
+      // stage, the stages' use parities and the key tile are carried along (no divisions in the loop)
+      int st = 0, kt = 0, n_st = kSolveStages;
+      uint32_t use_par = 0;  // bit st
       for (int i = 0; !ptx::c_withhold_loads; ++i) {
         if (i == total) {
           // the first sweeps are through: stream S again only if the row warps ask for it
@@ -233,7 +242,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           total = (third_sweep && !second) ? total_first + T_k : total_full + (third_sweep ? T_k : 0);
         }
         if (*cta_abort) break;
-        if (!ptx::mbar_wait(k_empty + st, use_par ^ 1)) {
+        if (!ptx::mbar_wait(k_empty + st, ((use_par >> st) & 1u) ^ 1u)) {
           raise_abort(cta_abort, p.status, kStTimeoutProducer);
           break;
         }
@@ -241,8 +250,9 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         for (int pn = 0; pn < PANELS; ++pn)
           ptx::tma_load_3d(sK + st * L::tile_bytes + pn * kPanelBytes, &tmK, k_full + st, pn * 64,
                            kt * kBlockN, kv_head);
-        if (++st == kSolveStages) { st = 0; use_par ^= 1; }
-        if (++kt == T_k) kt = 0;
+        use_par ^= 1u << st;
+        if (++kt == T_k) { kt = 0; n_st = late_stages; }
+        if (++st >= n_st) st = 0;
       }
     }
   } else if (warp == 17 || warp == 18) {
@@ -262,8 +272,8 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
       if (!ok) raise_abort(cta_abort, p.status, kStTimeoutMma);
       int total = total_first;
       // stage / key tile / number of the K tile's first product (and its buffer) are carried along
-      int st = 0, kt = 0, n0p = 0, bf0 = 0;
-      uint32_t k_par = 0, free_par = 0;  // bit b of free_par: parity of this issuer's next wait for buffer b
+      int st = 0, kt = 0, n_st = kSolveStages, n0p = 0, bf0 = 0;
+      uint32_t k_par = 0, free_par = 0;  // bit st of k_par, bit b of free_par: parity of this issuer's next wait for that stage / buffer
       const uint32_t a_tmem = tmem_base + kSolveQCol + g * (D / 2);
       for (int i = 0; ok; ++i) {
         if (i == total) {
@@ -274,7 +284,7 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           total = (third_sweep && !second) ? total_first + T_k : total_full + (third_sweep ? T_k : 0);
         }
         if (*cta_abort) break;
-        if (!ptx::mbar_wait(k_full + st, k_par)) { raise_abort(cta_abort, p.status, kStTimeoutMma); break; }
+        if (!ptx::mbar_wait(k_full + st, (k_par >> st) & 1u)) { raise_abort(cta_abort, p.status, kStTimeoutMma); break; }
         const int has_a = kt < T_a ? 1 : 0;  // the diagonal key tile of B has nothing for A
         if (g == 1 || has_a) {
           const int skip = g == 1 ? has_a : 0;  // B's product follows A's
@@ -304,8 +314,9 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
         n0p += adv;
         bf0 += adv;
         if (bf0 >= kSolveBufs) bf0 -= kSolveBufs;
-        if (++st == kSolveStages) { st = 0; k_par ^= 1; }
-        if (++kt == T_k) kt = 0;
+        k_par ^= 1u << st;
+        if (++kt == T_k) { kt = 0; n_st = late_stages; }
+        if (++st >= n_st) st = 0;
       }
     }
   } else {
@@ -691,6 +702,11 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
           thr_list = fmaxf(thr_list, hs.lo - 2e-5f);
           reset_stats();
         }
+      }
+      // once both row tiles are through with sweep 1 no product reads the last K stage any more, which
+      // is part of the pool from here on
+      if (late_stages < kSolveStages) ptx::bar_sync(3, kSolveRowThreads);
+      if (grp_on) {
         sweep_tiles(std::integral_constant<int, kModeCollect>{});
         if (lane == 0) pool_used[warp] = my_used;
         __syncwarp();
@@ -728,7 +744,10 @@ solve_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CU
       if (third_sweep && full_sweeps) {
         // ---- the lists of scores within 1 of the maximum did not fit: lists of the scores above
         // the histogram's lower bound, from one more sweep ----
-        if (threadIdx.x == 0) *pool_common = 0;
+        if (threadIdx.x == 0) {
+          *pool_common = 0;
+          if (p.sup_on) atomicAdd(p.sup.cursor + 4 + sup::kThirdSweep, 1u);
+        }
         head = kCandNil;
         ncand = 0;
         ptx::bar_sync(3, kSolveRowThreads);

@@ -26,7 +26,7 @@
 //
 // Layout of the support buffer (all offsets multiples of 256 bytes):
 //   [0]      uint32 cursor: entries handed out so far (one atomicAdd per solver CTA);
-//            words 4..7: solver CTAs that could not export, by reason (kWhy*)
+//            words 4..7: solver CTAs that could not export, by reason (kWhy*), or took a third sweep
 //   [256]    int32 dense[B*Hkv]
 //   kmax2    float [B*Hkv]: largest squared norm of a key row of the head (alpha > 1.5 only)
 //   rows     uint2 [B*Hq*N]: (index of the row's first entry, number of entries)
@@ -55,7 +55,7 @@ constexpr int kTableKeys = 32;      // keys per entry of the key-block table = k
 // why a solver CTA did not export (counters in words 4..7 of the buffer)
 enum : int {
   kWhyPool = 0,   // its candidate pool overflowed, in the third sweep as well (or a wait gave up)
-  kWhyUnused = 1,
+  kThirdSweep = 1,  // (not a failure: it took a third sweep)
   kWhyBlock = 2,  // more than kBlockCap entries in its 256 rows
   kWhyFull = 3,   // the entry array is full
 };
