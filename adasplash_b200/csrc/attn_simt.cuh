@@ -15,7 +15,8 @@
 // slots; the same fp32 arithmetic), and the tiles of fp32 inputs arrive by cp.async while the
 // product before them runs.  Row blocks are handed out heaviest first over all heads: a causal
 // problem of a few heads is as long as its last row block.  fp32, 8 heads of N = 2048, D = 64, unit
-// variance, forward and backward: 2.11 -> 0.96 ms (solver 619, forward 466, dQ 425, dK/dV 615 us before).
+// variance, forward and backward: 2.11 -> 0.96 ms (solver 619 -> 250,
+// forward 466 -> 217, dQ 425 -> 230, dK/dV 615 -> 287 us).
 #pragma once
 #include "common.cuh"
 

@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(kRowThreads) fwd_rows_kernel(RowsParams p) {
 // Largest squared norm of a key row per kv head (the solver's export needs it above alpha = 1.5
 // to bound the difference between the two roundings of a score).  Reads K once, 16 bytes per lane
 // with D/8 lanes on a row, and ends with one atomic per CTA of kNormRows rows.  Bound by HBM (or L2,
-// where the solver finds K again).
+// where the solver finds K again).  4 x 32 heads of 8192, D = 64 (134 MB): 25 us = 5.4 TB/s; a warp and an
+// atomic per row took 690.
 constexpr int kNormRows = 512;
 
 template <typename T, int D>
@@ -225,7 +226,8 @@ int fwd_t(const simt::Params& p, cudaStream_t st) {
   rp.B = p.B; rp.Hq = p.Hq; rp.Hkv = p.Hkv; rp.N = p.N; rp.Dg = p.D;
   rp.alpha = p.alpha;
   rp.sv = sup::view(p.support, nullptr, p.B, p.Hq, p.Hkv, p.N);
-  // fewer than four CTAs per SM at 32 rows per warp: eight rows per warp
+  // fewer than four CTAs per SM at 32 rows per warp: eight rows per warp (8 heads of 2048: 24 -> 11 us;
+  // 64 heads of 1500, which is 2.5 CTAs per SM: 66 -> 44 us)
   const bool small = (long long)p.B * p.Hq * p.N < 4LL * 148 * kRowsPerWarp * (kRowThreads / 32);
   const int rows_w = small ? 8 : kRowsPerWarp;
   const long long warps = (long long)p.B * p.Hq * ((p.N + rows_w - 1) / rows_w);
@@ -399,7 +401,8 @@ __global__ void __launch_bounds__(kBwdRowThreads) bwd_rows_kernel(BwdParams p) {
   // needs: it regroups by key, stably, itself): a stable counting sort.  Warp w of the sorting
   // warps takes the w-th stretch of the entries, counts its entries per key block, and -- after a
   // scan over (key block, warp) -- hands out their places in the same order.  (A bitonic network over
-  // (key, row) kept shared memory busy for 30 % of this kernel's time.)
+  // (key, row) kept shared memory busy: this kernel on 4 x 32 heads of 8192, 9 entries per row, 1397 ->
+  // 1069 us; on 8 x 32 heads of 4096 to 16384, 24 per row, 10.97 -> 6.86 ms.)
   __syncthreads();
   uint32_t total = 0;
 #pragma unroll
@@ -484,7 +487,8 @@ __global__ void __launch_bounds__(kBwdRowThreads) bwd_rows_kernel(BwdParams p) {
 // (head, row block, key, row), and a round fetches kStage of them to shared memory, each thread
 // looking up by bisection which segment its places belong to -- so that all loads of a round are in
 // flight together, however the entries are spread over segments.  (Copying segment by segment cost an L2
-// round trip per segment and warp: with 8 heads of 256 row blocks per key head, most of the kernel.)
+// round trip per segment and warp: 2 x 8 heads of 65536 on one key head 1943 -> 1250 us, 4 x 32 heads of 8192,
+// with few segments, 1061 -> 1014.)
 // The staged entries are regrouped by key with a stable counting sort.  The eight lanes of a
 // key then run through the key's range four entries at a time (the Q / dO rows of all four
 // requested before the first is used) and add P^T dO_i and dS^T Q_i.  No atomics: every sum has
