@@ -485,3 +485,22 @@ def test_fp32_solver_lists_and_sweeps(D, scale, N, vl):
             want[hit[:, 0], hit[:, 1] // 64, hit[:, 2] // 64] = True
             got = torch.stack([(bm[b, :, :N // 64, j // 32].cpu() >> (j % 32)) & 1 for j in range(N // 64)], -1).bool()
             assert (got | ~want).all() if must else (want | ~got).all()
+
+
+@pytest.mark.parametrize("D,scale,niter", [(64, 0.05, 2), (128, 0.05, 0), (128, 0.7, 3), (128, 1.5, 1)])
+def test_solver_of_long_ctas(D, scale, niter):
+    # More than 56 key tiles: the pool takes a K stage after the first sweep, and the sweeps that
+    # follow an overflow (flat rows) stream through the other two.  Against the CUDA-core solver, as in
+    # test_solver_with_nearly_flat_rows.
+    N, lens = 8192, [8192, 7300]
+    q = _randn((2, 1, N, D), 97, scale, torch.bfloat16).cuda()
+    k = _randn((2, 1, N, D), 98, 1.0, torch.bfloat16).cuda()
+    varlen = torch.tensor(lens, dtype=torch.int32).cuda()
+    _lib.set_kernel_path("simt")
+    tb, mb = att.solve(q, k, niter, varlen)
+    _lib.set_kernel_path("tcgen05")
+    for sup in (None, att.support_buffer(att.make_shape(q, k, niter, varlen), q.device)):
+        ta, ma = att.solve(q, k, niter, varlen, support=sup)
+        for b, n in enumerate(lens):
+            assert (ta[b, :, :n] - tb[b, :, :n]).abs().max() < (1e-4 if niter == 0 else 1e-5)
+        assert _popcount(ma ^ mb) <= 2 + _popcount(mb) // 1000   # scores within a rounding of tau
